@@ -1,10 +1,11 @@
 // Compile-time-class Rys ERI + J/K kernel for angular momenta up to d
 // (thread per contracted quartet, the quartet's work sliced over TPQ warps).
 //
-// Tile: a group of TPQ warps takes one bra shell pair and 32 consecutive ket
-// shell pairs of one primitive-count segment of the same class (one quartet
-// per lane); a CTA holds BBQ independent groups, each pulling chunks of
-// tiles from a launch counter.
+// Tile: a group of TPQ warps takes one bra shell pair and 32 / SPLIT
+// consecutive ket shell pairs of one primitive-count segment of the same
+// class (SPLIT lanes per quartet, one where the schedule fills the chip); a
+// CTA holds BBQ independent groups, each pulling chunks of tiles from a launch
+// counter.
 //
 // Phase 1 (registers): every thread of a quartet evaluates the primitive
 // loop (Rys roots/weights, 2-D VRR) and accumulates its own slice of the
@@ -12,6 +13,11 @@
 // NAS x NCS block, g = warp index inside the group.  The slice is fixed at
 // compile time, so the accumulators stay in registers; TPQ is the smallest
 // power of two whose slice holds at most fast_acc_limit() accumulators.
+// The lanes of a split quartet take the ket and bra primitives in strides and
+// add their accumulators by shuffles; the first of them goes on.  A deep contraction is one long dependent chain per
+// lane (about 0.2 us per primitive quartet in FP64): with one lane per quartet
+// and few tiles the whole launch waited for single warps (24-atom organic
+// molecule, (ss|ss): 8.2 ms for 0.5 ms worth of work).
 // Phase 2: ket HRR and ket spherical projection of the owned rows, written
 // to shared memory as (a0|cd)_sph rows.
 // Phase 3: after a barrier, each warp takes a share of the ket columns
@@ -205,10 +211,18 @@ struct QuartetGeom {
     double AB[3], CD[3];
 };
 
+// This lane's share of a quartet's primitive loops: ket primitives ik0,
+// ik0 + ikn, ..., bra primitives ib0, ib0 + ibn, ...; `lanes` lanes (a power
+// of two, neighbours in the warp) share the quartet.
+struct LaneSplit {
+    int ik0, ikn, ib0, ibn, lanes;
+};
+
 // Phase 1 + 2 for slice G (rows ia = G, G+TPQ, ...).
 template <typename R, int LA, int LB, int LC, int LD, int G>
 __device__ __forceinline__ void fast_slice(const PlanView& pv, int bra, int ket, bool active, const QuartetGeom& q,
-                                           double fs_thr2, const float* rtab, R* __restrict__ ks) {
+                                           const LaneSplit& sp, double fs_thr2, const float* rtab,
+                                           R* __restrict__ ks) {
     using S = FastShape<LA, LB, LC, LD>;
     constexpr int ROWS = (S::NAS - G + S::TPQ - 1) / S::TPQ;
     R acc[ROWS > 0 ? ROWS : 1][S::NCS];
@@ -236,7 +250,7 @@ __device__ __forceinline__ void fast_slice(const PlanView& pv, int bra, int ket,
         // Ket primitive outer, bra primitive inner: each lane gathers its own
         // ket record once per bra, and the bra records (the same for every
         // lane of the warp) are broadcast loads.
-        for (int ik = 0; ik < npk; ++ik) {
+        for (int ik = sp.ik0; ik < npk; ik += sp.ikn) {
             const double fsk = fs_on ? __ldg(pv.prim_fs + ok + ik) : 0.0;
             R qe, QCx, QCy, QCz, kw, kip;
             double kp_x = 0.0, kp_y = 0.0, kp_z = 0.0;
@@ -250,7 +264,7 @@ __device__ __forceinline__ void fast_slice(const PlanView& pv, int bra, int ket,
                 QCx = R(kp_x - q.C[0]); QCy = R(kp_y - q.C[1]); QCz = R(kp_z - q.C[2]);
                 kw = R(k2v.x); kip = R(k2v.y);
             }
-            for (int ib = 0; ib < npb; ++ib) {
+            for (int ib = sp.ib0; ib < npb; ib += sp.ibn) {
                 if (fs_on && !(__ldg(pv.prim_fs + ob + ib) * fsk >= fs_thr2)) continue;
                 R p, PAx, PAy, PAz, bw, bip, PQx, PQy, PQz;
                 if constexpr (F32) {
@@ -335,6 +349,14 @@ __device__ __forceinline__ void fast_slice(const PlanView& pv, int bra, int ket,
         }
     }
 
+    // Sum of a split quartet's lanes (the split is the same for the whole warp).
+    for (int o = 1; o < sp.lanes; o <<= 1) {
+#pragma unroll
+        for (int rr = 0; rr < ROWS; ++rr)
+#pragma unroll
+            for (int ic = 0; ic < S::NCS; ++ic) acc[rr][ic] += __shfl_xor_sync(0xffffffffu, acc[rr][ic], o);
+    }
+
     // Phase 2: ket transfer + projection of the owned rows (in R: the FP32
     // kernels keep the whole quartet in FP32 up to the FP64 atomics).
     const R CDr[3] = {R(q.CD[0]), R(q.CD[1]), R(q.CD[2])};
@@ -353,14 +375,14 @@ __device__ __forceinline__ void fast_slice(const PlanView& pv, int bra, int ket,
 
 template <typename R, int LA, int LB, int LC, int LD, int G = 0>
 __device__ __forceinline__ void fast_slice_dispatch(int g, const PlanView& pv, int bra, int ket, bool active,
-                                                    const QuartetGeom& q, double fs_thr2, const float* rtab,
-                                                    R* ks) {
+                                                    const QuartetGeom& q, const LaneSplit& sp, double fs_thr2,
+                                                    const float* rtab, R* ks) {
     using S = FastShape<LA, LB, LC, LD>;
     if constexpr (G < S::TPQ) {
         if (g == G)
-            fast_slice<R, LA, LB, LC, LD, G>(pv, bra, ket, active, q, fs_thr2, rtab, ks);
+            fast_slice<R, LA, LB, LC, LD, G>(pv, bra, ket, active, q, sp, fs_thr2, rtab, ks);
         else
-            fast_slice_dispatch<R, LA, LB, LC, LD, G + 1>(g, pv, bra, ket, active, q, fs_thr2, rtab, ks);
+            fast_slice_dispatch<R, LA, LB, LC, LD, G + 1>(g, pv, bra, ket, active, q, sp, fs_thr2, rtab, ks);
     }
 }
 
@@ -455,8 +477,11 @@ __global__ void __launch_bounds__(32 * FastShape<LA, LB, LC, LD>::WARPS, fast_mi
     const int ntiles = cl.tile_end - cl.tile_begin;
     double csum = 0.0;  // ERI checksum stream: this thread's share
 
-    // tiles per fetch (per-class tuning; 0 = the default)
-    const int chunk = cl.chunk > 0 ? cl.chunk : kTileChunk;
+    // Tiles per fetch (per-class tuning; 0 = the default): kTileChunk, fewer
+    // where a group would fetch less than 8 times in the whole launch, so that
+    // the last fetches of a small schedule are single tiles.
+    const int chunk = cl.chunk > 0 ? cl.chunk
+                                   : max(1, min(kTileChunk, ntiles / (8 * static_cast<int>(gridDim.x) * S::BBQ)));
     // Dynamic schedule: every warp group takes `chunk` consecutive tiles
     // (one bra pair x 32 kets each) from the launch counter, so all groups
     // work inside one moving window of the schedule and the density, J and
@@ -484,7 +509,11 @@ __global__ void __launch_bounds__(32 * FastShape<LA, LB, LC, LD>::WARPS, fast_mi
         }
         const int kb = tile - __ldg(cl.tile_prefix + b);
         const BlockDesc bd = cl.blocks[b];
-        const int j = kb * 32 + lane;
+        const int ls = bd.lk + bd.lb;
+        const int part = lane & ((1 << ls) - 1);
+        const LaneSplit sp{part & ((1 << bd.lk) - 1), 1 << bd.lk, part >> bd.lk, 1 << bd.lb, 1 << ls};
+        const bool digester = part == 0;
+        const int j = (kb * 32 + lane) >> ls;
         const bool lane_ok = j < bd.nket;
         const int ket = bd.ket0 + (lane_ok ? j : 0);
 
@@ -611,14 +640,16 @@ __global__ void __launch_bounds__(32 * FastShape<LA, LB, LC, LD>::WARPS, fast_mi
             else
                 any = __any_sync(0xffffffffu, active);
             if (!any) continue;
-            touched = touched || active;
+            touched = touched || (active && digester);
 
 #pragma unroll
             for (int k = 0; k < 3; ++k) {
                 q.A[k] = __ldg(pv.shell_xyz + 3 * A + k);
                 q.AB[k] = q.A[k] - __ldg(pv.shell_xyz + 3 * B + k);
             }
-            fast_slice_dispatch<R, LA, LB, LC, LD>(g, pv, bra, ket, active, q, cl.fs_thr2, rtab, ks);
+            fast_slice_dispatch<R, LA, LB, LC, LD>(g, pv, bra, ket, active, q, sp, cl.fs_thr2, rtab, ks);
+            // one lane of a split quartet digests it
+            active = active && digester;
             if constexpr (S::TPQ > 1) group_sync(bar_id, bar_n);
 
             // ---- bra transfer + projection per owned ket column, digestion ----
@@ -805,6 +836,8 @@ template <int LA, int LB, int LC, int LD>
 constexpr int fast_warps() { return FastShape<LA, LB, LC, LD>::WARPS; }
 template <int LA, int LB, int LC, int LD>
 constexpr int fast_bras() { return FastShape<LA, LB, LC, LD>::GB; }
+template <int LA, int LB, int LC, int LD>
+constexpr int fast_groups() { return FastShape<LA, LB, LC, LD>::BBQ; }
 template <int LA, int LB, int LC, int LD>
 constexpr int fast_smem_bytes() { return FastShape<LA, LB, LC, LD>::SMEM_DOUBLES * 8; }
 template <int LA, int LB, int LC, int LD>

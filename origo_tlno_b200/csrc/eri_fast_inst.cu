@@ -34,6 +34,7 @@ namespace tlno_gpu {
                              cudaFuncAttributeMaxDynamicSharedMemorySize, fast_smem_##id(true));        \
     }                                                                                                   \
     int fast_bras_##id() { return dev::fast_bras<a, b, c, d>(); }                                       \
+    int fast_groups_##id() { return dev::fast_groups<a, b, c, d>(); }                                   \
     int fast_blocks_per_sm_##id(bool fp32) {                                                            \
         constexpr int threads = 32 * dev::fast_warps<a, b, c, d>();                                     \
         int n = 0;                                                                                      \

@@ -4,6 +4,7 @@
 #include "kernels.hpp"
 
 #include <algorithm>
+#include <atomic>
 #include <cmath>
 #include <mutex>
 #include <set>
@@ -550,15 +551,12 @@ int fast_kernel_bras(int la, int lb, int lc, int ld) {
     }
 }
 
-bool launch_eri_jk_fast(const PlanView& pv, const ClassLaunch& cl, bool fp32, int grid, cudaStream_t s) {
-    const int idx = fast_class_index(cl.la, cl.lb, cl.lc, cl.ld);
-    if (idx < 0) return false;
-    if (cl.tile_end <= cl.tile_begin) return true;
-    const int ntiles = cl.tile_end - cl.tile_begin;
-    // One resident wave of persistent CTAs (a second partial wave would
-    // leave most SMs idle while it runs).
-    static int resident[TLNO_FAST_COUNT][2] = {};
-    int& nb = resident[idx][fp32 ? 1 : 0];
+// Resident CTAs per SM of a class's compile-time kernel (occupancy query,
+// remembered per class and precision).
+static int fast_resident(int idx, bool fp32) {
+    static std::atomic<int> resident[TLNO_FAST_COUNT][2];
+    std::atomic<int>& slot = resident[idx][fp32 ? 1 : 0];
+    int nb = slot.load(std::memory_order_relaxed);
     if (nb == 0) {
         switch (idx) {
 #define TLNO_FAST_OCC(id, a, b, c, d) \
@@ -567,7 +565,32 @@ bool launch_eri_jk_fast(const PlanView& pv, const ClassLaunch& cl, bool fp32, in
 #undef TLNO_FAST_OCC
             default: nb = 1;
         }
+        slot.store(nb, std::memory_order_relaxed);
     }
+    return nb;
+}
+
+int fast_kernel_resident_groups(int la, int lb, int lc, int ld) {
+    const int idx = fast_class_index(la, lb, lc, ld);
+    if (idx < 0) return 1;
+    int groups = 1;
+    switch (idx) {
+#define TLNO_FAST_GROUPS(id, a, b, c, d) \
+    case id: groups = fast_groups_##id(); break;
+        TLNO_FAST_CLASSES(TLNO_FAST_GROUPS)
+#undef TLNO_FAST_GROUPS
+    }
+    return sm_count() * fast_resident(idx, false) * groups;
+}
+
+bool launch_eri_jk_fast(const PlanView& pv, const ClassLaunch& cl, bool fp32, int grid, cudaStream_t s) {
+    const int idx = fast_class_index(cl.la, cl.lb, cl.lc, cl.ld);
+    if (idx < 0) return false;
+    if (cl.tile_end <= cl.tile_begin) return true;
+    const int ntiles = cl.tile_end - cl.tile_begin;
+    // One resident wave of persistent CTAs (a second partial wave would
+    // leave most SMs idle while it runs).
+    const int nb = fast_resident(idx, fp32);
     const int wave = sm_count() * nb;
     grid = (grid <= 0) ? wave : std::min(grid, wave);
     grid = std::min(grid, ntiles);

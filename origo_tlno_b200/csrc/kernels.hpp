@@ -33,6 +33,9 @@ bool has_fast_kernel(int la, int lb, int lc, int ld);
 // Bra pairs per CTA of the compile-time kernel of a class (its schedule's
 // block height).
 int fast_kernel_bras(int la, int lb, int lc, int ld);
+// Warp groups of the class's FP64 compile-time kernel resident on the device
+// (each works on one tile at a time).
+int fast_kernel_resident_groups(int la, int lb, int lc, int ld);
 
 void launch_onee(const dev::OneeLaunch& L, cudaStream_t s);
 // out = (X + X^T) / 2 for `count` stacked M x M blocks (offsets per block).

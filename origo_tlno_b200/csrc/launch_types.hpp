@@ -74,6 +74,10 @@ struct BlockDesc {
     int xbeg;      // first pair of the bra class list of this molecule
                    // (triangle test on the diagonal class: i = bra - xbeg)
     int koff;      // position of the segment inside the ket class list
+    // Lanes of one quartet (compile-time kernels): 2^lk lanes share the ket
+    // primitives and 2^lb the bra primitives, so a tile holds 32 >> (lk + lb)
+    // kets (rule: fast_tile_shape in plan.cpp).
+    int lk, lb;
 };
 
 // Quartet class and the schedule of one launch.

@@ -14,8 +14,11 @@
 #include "plan.hpp"
 
 #include <algorithm>
+#include <atomic>
 #include <cmath>
+#include <exception>
 #include <functional>
+#include <mutex>
 #include <numeric>
 #include <thread>
 
@@ -81,6 +84,59 @@ double flops_per_prim(int a, int b, int c, int d) {
     const double ncart4 = double(n_cart(a)) * n_cart(b) * n_cart(c) * n_cart(d);
     return 30.0 + N * (40.0 + 15.0 + 3.0 * vaxis + 3.0 * ncart4);
 }
+// ---- tile shapes of the compile-time kernels ----
+// Work of a tile beside its primitive loop (geometry, transfers, digestion), in
+// primitive-quartet steps.
+constexpr int kTileOverheadSteps = 8;
+
+// Serial steps a tile may take.  The dynamic schedule hands the heaviest tiles
+// out first, so a launch ends within one tile of the average load; a quarter of
+// a resident warp group's share keeps that tail small, and below 8 steps the
+// tile's own overhead outweighs a finer split.
+double fast_tile_limit(double class_steps, int resident_groups) {
+    return std::max(class_steps / (4.0 * std::max(resident_groups, 1)), double(kTileOverheadSteps));
+}
+
+// Bras per block and lanes per quartet (2^lk over the ket primitives, 2^lb over
+// the bra primitives) that keep a tile inside `limit` steps: fewer bras per
+// block first (that costs only shared sums), then lanes per quartet (that costs
+// idle lanes in the digestion), never more lanes than primitives.
+struct TileShape {
+    int bras, lk, lb;
+};
+TileShape fast_tile_shape(int npb, int npk, int nbra, double limit) {
+    TileShape t{nbra, 0, 0};
+    const double per_bra = double(npb) * npk + kTileOverheadSteps;
+    if (per_bra * nbra <= limit) return t;
+    t.bras = std::max(1, static_cast<int>(limit / per_bra));
+    if (t.bras > 1) return t;
+    while (t.lk + t.lb < 5 && double(npb) * npk / (1 << (t.lk + t.lb)) > limit) {
+        if ((2 << t.lk) <= npk) ++t.lk;
+        else if ((2 << t.lb) <= npb) ++t.lb;
+        else break;
+    }
+    return t;
+}
+
+// Reorders a schedule's blocks by falling cost (log2 of a tile's serial steps),
+// the order inside a cost kept, and rebuilds the tile prefix.
+void heaviest_first(std::vector<dev::BlockDesc>& blocks, std::vector<int>& prefix, const std::vector<int>& cost) {
+    // counting sort over the at most 32 cost values
+    std::array<std::size_t, 33> at{};
+    for (int c : cost) ++at[31 - c + 1];
+    for (std::size_t c = 1; c < at.size(); ++c) at[c] += at[c - 1];
+    std::vector<int> order(blocks.size());
+    for (std::size_t k = 0; k < blocks.size(); ++k) order[at[31 - cost[k]]++] = static_cast<int>(k);
+    std::vector<dev::BlockDesc> b(blocks.size());
+    std::vector<int> p(prefix.size(), 0);
+    for (std::size_t k = 0; k < order.size(); ++k) {
+        b[k] = blocks[order[k]];
+        p[k + 1] = p[k] + prefix[order[k] + 1] - prefix[order[k]];
+    }
+    blocks.swap(b);
+    prefix.swap(p);
+}
+
 // Per contracted quartet: 2 x projection terms + 12 per spherical ERI.
 double flops_per_contracted(int a, int b, int c, int d) {
     const double ncart4 = double(n_cart(a)) * n_cart(b) * n_cart(c) * n_cart(d);
@@ -438,12 +494,56 @@ void build_plan(Plan2e& plan, const std::vector<const Basis*>& bases, std::vecto
     upload_vec(plan.d_mol_ns, plan.mol_ns, s);
     upload_vec(plan.d_rho_off, plan.rho_off, s);
 
+    // Ket segments of every (molecule, pair class): runs of equal primitive
+    // count, with Q sorted descending inside a segment (exact quartet counts)
+    // and, per position, the largest Q of its bucket (non-increasing along the
+    // segment) for the schedule extent.
+    struct KetClass {
+        std::vector<int> seg;
+        std::vector<double> qsorted, bmax;
+    };
+    std::vector<KetClass> kets(static_cast<std::size_t>(plan.n_mol) * kMaxPairClasses);
+    for (int m = 0; m < plan.n_mol; ++m)
+        for (int Y = 0; Y < kMaxPairClasses; ++Y) {
+            const int nY = plan.mol_pairs[m].cls_count[Y];
+            if (nY == 0) continue;
+            const int by0 = gbeg[m][Y];
+            KetClass& kc = kets[static_cast<std::size_t>(m) * kMaxPairClasses + Y];
+            kc.seg.push_back(0);
+            for (int j = 1; j < nY; ++j)
+                if (plan.pair_nprim[by0 + j] != plan.pair_nprim[by0 + j - 1]) kc.seg.push_back(j);
+            kc.seg.push_back(nY);
+            const double* qk = plan.pair_Q.data() + by0;
+            kc.qsorted.assign(qk, qk + nY);
+            kc.bmax.resize(nY);
+            for (std::size_t sg = 0; sg + 1 < kc.seg.size(); ++sg) {
+                const int s0 = kc.seg[sg], s1 = kc.seg[sg + 1];
+                std::sort(kc.qsorted.begin() + s0, kc.qsorted.begin() + s1, std::greater<double>());
+                for (int j = s0; j < s1;) {
+                    int e = j;
+                    double mx = 0.0;
+                    const int bk = Q_bucket(qk[j]);
+                    while (e < s1 && Q_bucket(qk[e]) == bk) mx = std::max(mx, qk[e++]);
+                    for (int t = j; t < e; ++t) kc.bmax[t] = mx;
+                    j = e;
+                }
+            }
+        }
+
     // Quartet-class schedules.
     plan.combos.clear();
     plan.total_quartets = plan.total_prim_quartets = 0;
     plan.total_flops = 0.0;
-    for (int X = 0; X < kMaxPairClasses; ++X) {
+    // The class schedules are independent: built on host threads, uploaded in
+    // class order.
+    std::vector<ComboSchedule> todo;
+    std::vector<int> resident;  // per class: warp groups on the device
+    for (int X = 0; X < kMaxPairClasses; ++X)
         for (int Y = 0; Y <= X; ++Y) {
+            bool any = false;
+            for (int m = 0; m < plan.n_mol && !any; ++m)
+                any = plan.mol_pairs[m].cls_count[X] > 0 && plan.mol_pairs[m].cls_count[Y] > 0;
+            if (!any) continue;
             ComboSchedule cs;
             cs.X = X;
             cs.Y = Y;
@@ -458,152 +558,204 @@ void build_plan(Plan2e& plan, const std::vector<const Basis*>& bases, std::vecto
                       !(combo_id < 256 && tune.force_generic[combo_id]);
             cs.bb = cs.fast ? fast_kernel_bras(cs.la, cs.lb, cs.lc, cs.ld) : 1;
             cs.bk = cs.fast ? 32 : tune.generic_bk;
-            const double fprim = flops_per_prim(cs.la, cs.lb, cs.lc, cs.ld);
-            const double fcon = flops_per_contracted(cs.la, cs.lb, cs.lc, cs.ld);
-            cs.prefix.push_back(0);
+            todo.push_back(std::move(cs));
+            resident.push_back(todo.back().fast ? fast_kernel_resident_groups(todo.back().la, todo.back().lb,
+                                                                              todo.back().lc, todo.back().ld)
+                                                : 1);
+        }
+    auto build_schedule = [&](ComboSchedule& cs, int resident_groups) {
+        const int X = cs.X, Y = cs.Y;
+        const double fprim = flops_per_prim(cs.la, cs.lb, cs.lc, cs.ld);
+        const double fcon = flops_per_contracted(cs.la, cs.lb, cs.lc, cs.ld);
+        // Tile extent of segment [s0, s1) for a bra of bound qi: the whole
+        // buckets that may hold a passing ket (on the diagonal class only
+        // local index <= i).
+        auto seg_extent = [&](const KetClass& kc, double qi, int s0, int s1, int i) {
+            int lo = s1;
+            if (tau > 0.0) {
+                lo = s0;
+                int hi = s1;
+                while (lo < hi) {
+                    const int mid = (lo + hi) / 2;
+                    if (qi * kc.bmax[mid] >= tau) lo = mid + 1; else hi = mid;
+                }
+            }
+            int e = lo - s0;
+            if (X == Y) e = std::min(e, i + 1 - s0);
+            return std::max(e, 0);
+        };
+        // Serial steps a tile may take (fast_tile_limit): from the steps of
+        // the whole class with one lane per quartet, sampled over the bras.
+        double limit = 1e300;
+        if (cs.fast) {
+            double steps = 0.0;
             for (int m = 0; m < plan.n_mol; ++m) {
-                const MolPairs& mp = plan.mol_pairs[m];
-                const int nX = mp.cls_count[X], nY = mp.cls_count[Y];
-                if (nX == 0 || nY == 0) continue;
-                const int bx0 = gbeg[m][X], by0 = gbeg[m][Y];
-                // ket segments of equal primitive count
-                std::vector<int> seg{0};
-                for (int j = 1; j < nY; ++j)
-                    if (plan.pair_nprim[by0 + j] != plan.pair_nprim[by0 + j - 1]) seg.push_back(j);
-                seg.push_back(nY);
-                const double* qk = plan.pair_Q.data() + by0;
-                // Per segment: Q sorted descending (exact quartet counts) and,
-                // per position, the largest Q of its bucket (non-increasing
-                // along the segment) for the schedule extent.
-                std::vector<double> qsorted(qk, qk + nY), bmax(nY);
+                const int nX = plan.mol_pairs[m].cls_count[X];
+                if (nX == 0 || plan.mol_pairs[m].cls_count[Y] == 0) continue;
+                const KetClass& kc = kets[static_cast<std::size_t>(m) * kMaxPairClasses + Y];
+                const int stride = std::max(1, nX / 1024);
+                for (int i = 0; i < nX; i += stride)
+                    for (std::size_t sg = 0; sg + 1 < kc.seg.size(); ++sg) {
+                        const int ext = seg_extent(kc, plan.pair_Q[gbeg[m][X] + i], kc.seg[sg], kc.seg[sg + 1], i);
+                        const int npk = plan.pair_nprim[gbeg[m][Y] + kc.seg[sg]];
+                        steps += stride * double((ext + 31) / 32) *
+                                 (double(plan.pair_nprim[gbeg[m][X] + i]) * npk + kTileOverheadSteps);
+                    }
+            }
+            limit = fast_tile_limit(steps, resident_groups);
+        }
+        cs.prefix.push_back(0);
+        std::vector<int> cost;  // per block: log2 of its tiles' serial steps
+        for (int m = 0; m < plan.n_mol; ++m) {
+            const MolPairs& mp = plan.mol_pairs[m];
+            const int nX = mp.cls_count[X], nY = mp.cls_count[Y];
+            if (nX == 0 || nY == 0) continue;
+            const int bx0 = gbeg[m][X], by0 = gbeg[m][Y];
+            const KetClass& kc = kets[static_cast<std::size_t>(m) * kMaxPairClasses + Y];
+            const std::vector<int>& seg = kc.seg;
+            // passing kets of segment [s0, s1) for a bra of bound qi
+            auto seg_count = [&](double qi, int s0, int s1) {
+                if (tau <= 0.0) return s1 - s0;
+                int a = s0, b = s1;
+                while (a < b) {
+                    const int mid = (a + b) / 2;
+                    if (qi * kc.qsorted[mid] >= tau) a = mid + 1; else b = mid;
+                }
+                return a - s0;
+            };
+            // Exact surviving quartets and primitive quartets.  Off the
+            // diagonal every (bra, ket) pair counts; on the diagonal class
+            // (one list, j <= i) a ket segment before the bra's segment
+            // counts fully and the bra's own segment holds
+            // (ordered pairs + self pairs) / 2.
+            {
+                std::vector<int> seg_of(nX);
+                if (X == Y)
+                    for (std::size_t sg = 0; sg + 1 < seg.size(); ++sg)
+                        for (int j = seg[sg]; j < seg[sg + 1]; ++j) seg_of[j] = static_cast<int>(sg);
+                std::vector<long long> own_ordered(seg.size(), 0), own_self(seg.size(), 0);
+                for (int i = 0; i < nX; ++i) {
+                    const double qi = plan.pair_Q[bx0 + i];
+                    const long long npb = plan.pair_nprim[bx0 + i];
+                    for (std::size_t sg = 0; sg + 1 < seg.size(); ++sg) {
+                        if (X == Y && static_cast<int>(sg) > seg_of[i]) break;
+                        const int c = seg_count(qi, seg[sg], seg[sg + 1]);
+                        if (X == Y && static_cast<int>(sg) == seg_of[i]) {
+                            own_ordered[sg] += c;
+                            if (tau <= 0.0 || qi * qi >= tau) own_self[sg] += 1;
+                            continue;
+                        }
+                        cs.quartets += c;
+                        cs.prim_quartets += npb * plan.pair_nprim[by0 + seg[sg]] * c;
+                    }
+                }
+                if (X == Y)
+                    for (std::size_t sg = 0; sg + 1 < seg.size(); ++sg) {
+                        const long long n = (own_ordered[sg] + own_self[sg]) / 2;
+                        const long long np = plan.pair_nprim[by0 + seg[sg]];
+                        cs.quartets += n;
+                        cs.prim_quartets += np * np * n;
+                    }
+            }
+            // Bra order: the class list order, or (bra groups) grouped by
+            // first shell A inside each primitive-count group, list order
+            // kept inside a group; a block holds up to cs.bb bras of one A,
+            // fewer where their serial steps pass the limit.
+            std::vector<int> order(nX);
+            for (int i = 0; i < nX; ++i) order[i] = i;
+            if (cs.bb > 1)
+                std::stable_sort(order.begin(), order.end(), [&](int u, int v) {
+                    const int nu = plan.pair_nprim[bx0 + u], nv = plan.pair_nprim[bx0 + v];
+                    if (nu != nv) return nu < nv;
+                    return plan.pair_A[bx0 + u] < plan.pair_A[bx0 + v];
+                });
+            for (int i0 = 0; i0 < nX;) {
+                int nbra = 1, npb = plan.pair_nprim[bx0 + order[i0]];
+                if (cs.bb > 1)
+                    while (nbra < cs.bb && i0 + nbra < nX &&
+                           plan.pair_A[bx0 + order[i0 + nbra]] == plan.pair_A[bx0 + order[i0]]) {
+                        npb = std::max(npb, plan.pair_nprim[bx0 + order[i0 + nbra]]);
+                        ++nbra;
+                    }
+                const int brabeg = static_cast<int>(cs.bra_list.size());
+                bool used = false;
                 for (std::size_t sg = 0; sg + 1 < seg.size(); ++sg) {
                     const int s0 = seg[sg], s1 = seg[sg + 1];
-                    std::sort(qsorted.begin() + s0, qsorted.begin() + s1, std::greater<double>());
-                    for (int j = s0; j < s1;) {
-                        int e = j;
-                        double mx = 0.0;
-                        const int bk = Q_bucket(qk[j]);
-                        while (e < s1 && Q_bucket(qk[e]) == bk) mx = std::max(mx, qk[e++]);
-                        for (int t = j; t < e; ++t) bmax[t] = mx;
-                        j = e;
-                    }
-                }
-                // Tile extent of segment [s0, s1) for a bra of bound qi: the
-                // whole buckets that may hold a passing ket (on the diagonal
-                // class only local index <= i).
-                auto seg_extent = [&](double qi, int s0, int s1, int i) {
-                    int lo = s1;
-                    if (tau > 0.0) {
-                        lo = s0;
-                        int hi = s1;
-                        while (lo < hi) {
-                            const int mid = (lo + hi) / 2;
-                            if (qi * bmax[mid] >= tau) lo = mid + 1; else hi = mid;
-                        }
-                    }
-                    int e = lo - s0;
-                    if (X == Y) e = std::min(e, i + 1 - s0);
-                    return std::max(e, 0);
-                };
-                // passing kets of segment [s0, s1) for a bra of bound qi
-                auto seg_count = [&](double qi, int s0, int s1) {
-                    if (tau <= 0.0) return s1 - s0;
-                    int a = s0, b = s1;
-                    while (a < b) {
-                        const int mid = (a + b) / 2;
-                        if (qi * qsorted[mid] >= tau) a = mid + 1; else b = mid;
-                    }
-                    return a - s0;
-                };
-                // Exact surviving quartets and primitive quartets.  Off the
-                // diagonal every (bra, ket) pair counts; on the diagonal class
-                // (one list, j <= i) a ket segment before the bra's segment
-                // counts fully and the bra's own segment holds
-                // (ordered pairs + self pairs) / 2.
-                {
-                    std::vector<int> seg_of(nX);
-                    if (X == Y)
-                        for (std::size_t sg = 0; sg + 1 < seg.size(); ++sg)
-                            for (int j = seg[sg]; j < seg[sg + 1]; ++j) seg_of[j] = static_cast<int>(sg);
-                    std::vector<long long> own_ordered(seg.size(), 0), own_self(seg.size(), 0);
-                    for (int i = 0; i < nX; ++i) {
-                        const double qi = plan.pair_Q[bx0 + i];
-                        const long long npb = plan.pair_nprim[bx0 + i];
-                        for (std::size_t sg = 0; sg + 1 < seg.size(); ++sg) {
-                            if (X == Y && static_cast<int>(sg) > seg_of[i]) break;
-                            const int c = seg_count(qi, seg[sg], seg[sg + 1]);
-                            if (X == Y && static_cast<int>(sg) == seg_of[i]) {
-                                own_ordered[sg] += c;
-                                if (tau <= 0.0 || qi * qi >= tau) own_self[sg] += 1;
-                                continue;
-                            }
-                            cs.quartets += c;
-                            cs.prim_quartets += npb * plan.pair_nprim[by0 + seg[sg]] * c;
-                        }
-                    }
-                    if (X == Y)
-                        for (std::size_t sg = 0; sg + 1 < seg.size(); ++sg) {
-                            const long long n = (own_ordered[sg] + own_self[sg]) / 2;
-                            const long long np = plan.pair_nprim[by0 + seg[sg]];
-                            cs.quartets += n;
-                            cs.prim_quartets += np * np * n;
-                        }
-                }
-                // Bra order: the class list order, or (bra groups) grouped by
-                // first shell A inside each primitive-count group, list order
-                // kept inside a group; a block holds up to cs.bb bras of one A.
-                std::vector<int> order(nX);
-                for (int i = 0; i < nX; ++i) order[i] = i;
-                if (cs.bb > 1)
-                    std::stable_sort(order.begin(), order.end(), [&](int u, int v) {
-                        const int nu = plan.pair_nprim[bx0 + u], nv = plan.pair_nprim[bx0 + v];
-                        if (nu != nv) return nu < nv;
-                        return plan.pair_A[bx0 + u] < plan.pair_A[bx0 + v];
-                    });
-                for (int i0 = 0; i0 < nX;) {
-                    int nbra = 1;
-                    if (cs.bb > 1)
-                        while (nbra < cs.bb && i0 + nbra < nX &&
-                               plan.pair_A[bx0 + order[i0 + nbra]] == plan.pair_A[bx0 + order[i0]])
-                            ++nbra;
-                    const int brabeg = static_cast<int>(cs.bra_list.size());
-                    bool used = false;
-                    for (std::size_t sg = 0; sg + 1 < seg.size(); ++sg) {
-                        const int s0 = seg[sg], s1 = seg[sg + 1];
+                    const int npk = plan.pair_nprim[by0 + s0];
+                    const TileShape ts = cs.fast ? fast_tile_shape(npb, npk, nbra, limit) : TileShape{1, 0, 0};
+                    const int bk = cs.bk >> (ts.lk + ts.lb);
+                    for (int w0 = 0; w0 < nbra; w0 += ts.bras) {
+                        const int w1 = std::min(nbra, w0 + ts.bras);
                         int ext = 0;
-                        for (int w = 0; w < nbra; ++w) {
+                        for (int w = w0; w < w1; ++w) {
                             const int i = order[i0 + w];
-                            ext = std::max(ext, seg_extent(plan.pair_Q[bx0 + i], s0, s1, i));
+                            ext = std::max(ext, seg_extent(kc, plan.pair_Q[bx0 + i], s0, s1, i));
                         }
-                        const int nt = (ext + cs.bk - 1) / cs.bk;
+                        const int nt = (ext + bk - 1) / bk;
                         if (nt <= 0) continue;
                         used = true;
                         dev::BlockDesc bd{};
-                        bd.bra0 = brabeg;
-                        bd.nbra = nbra;
+                        bd.bra0 = brabeg + w0;
+                        bd.nbra = w1 - w0;
                         bd.ket0 = by0 + s0;
                         bd.nket = s1 - s0;
                         bd.xbeg = bx0;
                         bd.koff = s0;
+                        bd.lk = ts.lk;
+                        bd.lb = ts.lb;
                         cs.blocks.push_back(bd);
                         cs.prefix.push_back(cs.prefix.back() + nt);
+                        int lg = 0;
+                        while ((npb * npk * (w1 - w0) >> (ts.lk + ts.lb)) >> (lg + 1)) ++lg;
+                        cost.push_back(lg);
                     }
-                    if (used)
-                        for (int w = 0; w < nbra; ++w) cs.bra_list.push_back(bx0 + order[i0 + w]);
-                    i0 += nbra;
                 }
+                if (used)
+                    for (int w = 0; w < nbra; ++w) cs.bra_list.push_back(bx0 + order[i0 + w]);
+                i0 += nbra;
             }
-            cs.n_tiles = cs.prefix.back();
-            if (cs.n_tiles == 0) continue;
-            cs.flops = fprim * cs.prim_quartets + fcon * cs.quartets;
-            upload_vec(cs.d_blocks, cs.blocks, s);
-            upload_vec(cs.d_prefix, cs.prefix, s);
-            upload_vec(cs.d_bra_list, cs.bra_list, s);
-            plan.total_quartets += cs.quartets;
-            plan.total_prim_quartets += cs.prim_quartets;
-            plan.total_flops += cs.flops;
-            plan.combos.push_back(std::move(cs));
         }
+        cs.n_tiles = cs.prefix.back();
+        if (cs.n_tiles == 0) return;
+        heaviest_first(cs.blocks, cs.prefix, cost);
+        cs.flops = fprim * cs.prim_quartets + fcon * cs.quartets;
+    };
+    {
+        // one class at a time per thread (the first exception is rethrown
+        // here); small plans are not worth a thread
+        std::atomic<std::size_t> next{0};
+        std::mutex mtx;
+        std::exception_ptr failed;
+        auto work = [&] {
+            try {
+                for (std::size_t k; (k = next.fetch_add(1)) < todo.size();) build_schedule(todo[k], resident[k]);
+            } catch (...) {
+                std::lock_guard<std::mutex> lock(mtx);
+                if (!failed) failed = std::current_exception();
+            }
+        };
+        const std::size_t nt = plan.kept_pairs < 2000
+                                   ? 1
+                                   : std::min<std::size_t>({std::max(1u, std::thread::hardware_concurrency()), 16,
+                                                            todo.size()});
+        std::vector<std::thread> threads;
+        try {
+            for (std::size_t t = 1; t < nt; ++t) threads.emplace_back(work);
+        } catch (...) {  // no more threads: the ones that started and this one do the work
+        }
+        work();
+        for (auto& t : threads) t.join();
+        if (failed) std::rethrow_exception(failed);
+    }
+    for (ComboSchedule& cs : todo) {
+        if (cs.n_tiles == 0) continue;
+        upload_vec(cs.d_blocks, cs.blocks, s);
+        upload_vec(cs.d_prefix, cs.prefix, s);
+        upload_vec(cs.d_bra_list, cs.bra_list, s);
+        plan.total_quartets += cs.quartets;
+        plan.total_prim_quartets += cs.prim_quartets;
+        plan.total_flops += cs.flops;
+        plan.combos.push_back(std::move(cs));
     }
     plan.d_counters.alloc(sizeof(int) * 2 * std::max<std::size_t>(plan.combos.size(), 1));
 
