@@ -23,6 +23,7 @@ struct DevTables {
     // contiguous 80N-byte record (40N bytes in FP32).
     const double* rys_h[kMaxRoots + 1];
     const float* rys_h32[kMaxRoots + 1];
+    const double* rys_raw1;         // N = 1 grid rows {root, weight}
     double tmax[kMaxRoots + 1];
     double h2[kMaxRoots + 1][kMaxRoots];
     double hw[kMaxRoots + 1][kMaxRoots];
@@ -158,24 +159,57 @@ __device__ __forceinline__ void rys_root(int N, R T, int i, R& root, R& weight) 
     weight = w;
 }
 
+// 1/sqrt(x) of a positive normal x: the hardware approximation y and one
+// third-order step y (1 + e/2 + 3 e^2/8), e = 1 - x y^2 (Householder's method),
+// 5 FP64 operations and no special-case branch.  With the asymptotic form built
+// on it (one rsqrt_pos instead of a division and a square root), which most warps
+// run for some lane: six light classes of 91 waters FP64 208 -> 184 ms, FP32
+// 138 -> 118 ms.
+__device__ __forceinline__ double rsqrt_pos(double x) {
+    double y;
+    asm("rsqrt.approx.ftz.f64 %0, %1;" : "=d"(y) : "d"(x));
+    const double e = fma(-x * y, y, 1.0);
+    return fma(fma(0.375, e, 0.5), y * e, y);
+}
+__device__ __forceinline__ float rsqrt_pos(float x) {
+    float y;
+    asm("rsqrt.approx.ftz.f32 %0, %1;" : "=f"(y) : "f"(x));
+    return y;
+}
+
+// Asymptotic Rys roots and weights (T >= tmax(N)).
+template <typename R, int N>
+__device__ __forceinline__ void rys_asymptotic(R T, R* root, R* weight) {
+    const R x = fmin(T, sizeof(R) == 4 ? R(1e37) : R(1e300));
+    const R s = rsqrt_pos(x);
+    R inv = s * s;
+    inv = fma(inv, fma(-x, inv, R(1)), inv);
+#pragma unroll
+    for (int i = 0; i < N; ++i) {
+        root[i] = R(c_tabs.h2[N][i]) * inv;
+        weight[i] = R(c_tabs.hw[N][i]) * s;
+    }
+}
+
 // All N roots at once (compile-time N).
+// FP64 N = 1 reads the interpolation's own grid values (rows of root and weight,
+// 46 KB, which stay in L1) and weights them by the 5-point Lagrange basis, the
+// same interpolant as the power-form records (232 KB): 20 more FP64 operations
+// for L1 instead of L2 latency, (ps|ss) of 91 waters without digestion 37.7 ->
+// 34.6 ms.  N = 2, 3 (118, 206 KB of rows) gained nothing and keep the records.
 template <typename R, int N>
 __device__ __forceinline__ void rys_roots_all(R T, R* root, R* weight) {
     if (T >= R(c_tabs.tmax[N])) {
-        const R inv = R(1) / T;
-        const R sinv = sqrt(inv);
-#pragma unroll
-        for (int i = 0; i < N; ++i) {
-            root[i] = R(c_tabs.h2[N][i]) * inv;
-            weight[i] = R(c_tabs.hw[N][i]) * sinv;
-        }
+        rys_asymptotic<R, N>(T, root, weight);
         return;
     }
     using V2 = typename RysTab<R>::V2;
     const R fi = T * R(100);
     const int k = static_cast<int>(fi);
     const R t = fi - R(k);
-    const V2* rec = reinterpret_cast<const V2*>(RysTab<R>::h(N) + static_cast<long long>(k) * 10 * N);
+    constexpr bool RAW = sizeof(R) == 8 && N == 1;
+    const V2* rec = RAW ? reinterpret_cast<const V2*>(c_tabs.rys_raw1) + k
+                        : reinterpret_cast<const V2*>(RysTab<R>::h(N)) + k * (5 * N);
     R c[5][2 * N];
 #pragma unroll
     for (int j = 0; j < 5; ++j)
@@ -185,14 +219,29 @@ __device__ __forceinline__ void rys_roots_all(R T, R* root, R* weight) {
             c[j][2 * m] = v.x;
             c[j][2 * m + 1] = v.y;
         }
+    if constexpr (RAW) {
+        const R u = t - R(2), s = u * u, A = s - R(1), B = s - R(4);
+        const R ua = (u * R(1.0 / 24.0)) * A, ub = (u * R(-1.0 / 6.0)) * B, ua2 = ua + ua;
+        const R l0 = ua * u - ua2, l1 = ub * u - ub, l2 = (R(0.25) * A) * B, l3 = ub * u + ub, l4 = ua * u + ua2;
 #pragma unroll
-    for (int i = 0; i < 2 * N; ++i) {
-        R v = c[4][i];
-        v = v * t + c[3][i];
-        v = v * t + c[2][i];
-        v = v * t + c[1][i];
-        v = v * t + c[0][i];
-        if (i < N) root[i] = v; else weight[i - N] = v;
+        for (int i = 0; i < 2 * N; ++i) {
+            R v = c[4][i] * l4;
+            v = v + c[0][i] * l0;
+            v = v + c[3][i] * l3;
+            v = v + c[1][i] * l1;
+            v = v + c[2][i] * l2;
+            if (i < N) root[i] = v; else weight[i - N] = v;
+        }
+    } else {
+#pragma unroll
+        for (int i = 0; i < 2 * N; ++i) {
+            R v = c[4][i];
+            v = v * t + c[3][i];
+            v = v * t + c[2][i];
+            v = v * t + c[1][i];
+            v = v * t + c[0][i];
+            if (i < N) root[i] = v; else weight[i - N] = v;
+        }
     }
 }
 
@@ -203,13 +252,7 @@ template <int N>
 __device__ __forceinline__ void rys_roots_smem32(float T, const float* __restrict__ table, float* root,
                                                  float* weight) {
     if (T >= float(c_tabs.tmax[N])) {
-        const float inv = 1.0f / T;
-        const float sinv = sqrtf(inv);
-#pragma unroll
-        for (int i = 0; i < N; ++i) {
-            root[i] = float(c_tabs.h2[N][i]) * inv;
-            weight[i] = float(c_tabs.hw[N][i]) * sinv;
-        }
+        rys_asymptotic<float, N>(T, root, weight);
         return;
     }
     const float x = T * float(kRys32PerUnitDev);

@@ -281,7 +281,7 @@ __device__ __forceinline__ void fast_slice(const PlanView& pv, int bra, int ket,
                 }
                 const R pqs = p + qe;
                 // one reciprocal square root gives both 1/sqrt(p+q) and 1/(p+q)
-                const R rs = rsqrt(pqs);
+                const R rs = rsqrt_pos(pqs);
                 const R inv = rs * rs;
                 const R Targ = p * qe * inv * (PQx * PQx + PQy * PQy + PQz * PQz);
                 R rt[S::N], wt[S::N];

@@ -659,29 +659,34 @@ __device__ void generic_quartet_cta(const PlanView& pv, const ClassLaunch& cl, c
 }
 
 // Tiled schedule (J/K mode), one quartet per block at a time: tile = 1 bra
-// pair x bk ket pairs, tiles handed out by a block-wide dynamic counter.
+// pair x bk ket pairs, handed out by a block-wide dynamic counter in parts of
+// `part` kets.  A quartet of two f shells takes a block 10-50 us, so whole
+// tiles of 64 left most SMs idle on small molecules (f-shell 14 atoms,
+// (ff|ff): 31 tiles, 393 quartets, 1.66 ms).
 template <typename R>
-__global__ void eri_generic_cta_jk_kernel(PlanView pv, ClassLaunch cl, int nb_items) {
+__global__ void eri_generic_cta_jk_kernel(PlanView pv, ClassLaunch cl, int nb_items, int part) {
     extern __shared__ double smem[];
     GenericCtaLayout lay;
     lay.init(cl.la, cl.lb, cl.lc, cl.ld, nb_items);
     __shared__ int s_tile;
     const double thr = (cl.prec_mode != 0) ? cl.tau_mix / fmax(*cl.dmax, 1e-300) : 0.0;
-    const int ntiles = cl.tile_end - cl.tile_begin;
+    const int parts = (cl.bk + part - 1) / part;
+    const int nunits = (cl.tile_end - cl.tile_begin) * parts;
     for (;;) {
         if (threadIdx.x == 0) s_tile = atomicAdd(cl.counter, 1);
         __syncthreads();
         const int t = s_tile;
         __syncthreads();
-        if (t >= ntiles) break;
-        const int tile = cl.tile_begin + t;
+        if (t >= nunits) break;
+        const int tile = cl.tile_begin + t / parts;
+        const int j0 = t % parts * part;
         const int b = find_block(cl.tile_prefix, cl.n_blocks, tile);
         const int kb = tile - __ldg(cl.tile_prefix + b);
         const BlockDesc bd = cl.blocks[b];
         const int bra = __ldg(cl.bra_list + bd.bra0);  // one bra per block
         const int i = bra - bd.xbeg;
         const double qi = pv.pair_Q[bra];
-        for (int jj = 0; jj < cl.bk; ++jj) {
+        for (int jj = j0; jj < min(j0 + part, cl.bk); ++jj) {
             const int j = kb * cl.bk + jj;
             if (j >= bd.nket) break;
             if (cl.same && bd.koff + j > i) break;

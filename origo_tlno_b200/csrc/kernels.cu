@@ -415,6 +415,14 @@ void ensure_device_tables() {
         const std::vector<double> rec = rys_power_records(h, n);
         t.rys_h[n] = upload(rec);
         t.rys_h32[n] = upload(std::vector<float>(rec.begin(), rec.end()));
+        if (n == 1) {
+            std::vector<double> rows;
+            for (int r = 0; r < h.rys_rows[1]; ++r) {
+                rows.push_back(h.rys_roots[1][r]);
+                rows.push_back(h.rys_weights[1][r]);
+            }
+            t.rys_raw1 = upload(rows);
+        }
         t.tmax[n] = h.rys_tmax[n];
         for (int i = 0; i < n; ++i) {
             t.h2[n][i] = h.herm_root2[n][i];
@@ -517,12 +525,17 @@ void launch_eri_jk_generic(const PlanView& pv, const ClassLaunch& cl, bool fp32,
         } else {
             TLNO_CUDA(cudaOccupancyMaxActiveBlocksPerMultiprocessor(&per_sm, eri_generic_cta_jk_kernel<double>, threads, bytes));
         }
-        const int ntiles = cl.tile_end - cl.tile_begin;
-        const int g = std::max(1, std::min(ntiles, sm_count() * std::max(per_sm, 1)));
+        const long long ntiles = cl.tile_end - cl.tile_begin;
+        const int wave = sm_count() * std::max(per_sm, 1);
+        // kets per fetch: a whole tile where every block fetches at least 16
+        // times, halved down to one quartet where the schedule is smaller
+        int part = cl.bk;
+        while (part > 1 && ntiles * ((cl.bk + part - 1) / part) < 16LL * wave) part = (part + 1) / 2;
+        const int g = static_cast<int>(std::max(1LL, std::min<long long>(ntiles * ((cl.bk + part - 1) / part), wave)));
         if (fp32)
-            eri_generic_cta_jk_kernel<float><<<g, threads, bytes, s>>>(pv, cl, nb_items);
+            eri_generic_cta_jk_kernel<float><<<g, threads, bytes, s>>>(pv, cl, nb_items, part);
         else
-            eri_generic_cta_jk_kernel<double><<<g, threads, bytes, s>>>(pv, cl, nb_items);
+            eri_generic_cta_jk_kernel<double><<<g, threads, bytes, s>>>(pv, cl, nb_items, part);
         TLNO_CUDA(cudaGetLastError());
         return;
     }
