@@ -23,7 +23,6 @@ struct DevTables {
     // contiguous 80N-byte record (40N bytes in FP32).
     const double* rys_h[kMaxRoots + 1];
     const float* rys_h32[kMaxRoots + 1];
-    const double* rys_raw1;         // N = 1 grid rows {root, weight}
     double tmax[kMaxRoots + 1];
     double h2[kMaxRoots + 1][kMaxRoots];
     double hw[kMaxRoots + 1][kMaxRoots];
@@ -181,7 +180,8 @@ __device__ __forceinline__ float rsqrt_pos(float x) {
 template <typename R, int N>
 __device__ __forceinline__ void rys_asymptotic(R T, R* root, R* weight) {
     const R x = fmin(T, sizeof(R) == 4 ? R(1e37) : R(1e300));
-    const R s = rsqrt_pos(x);
+    R s = rsqrt_pos(x);
+    if (sizeof(R) == 4) s = fma(R(0.5) * s, fma(-x * s, s, R(1)), s);
     R inv = s * s;
     inv = fma(inv, fma(-x, inv, R(1)), inv);
 #pragma unroll
@@ -192,11 +192,6 @@ __device__ __forceinline__ void rys_asymptotic(R T, R* root, R* weight) {
 }
 
 // All N roots at once (compile-time N).
-// FP64 N = 1 reads the interpolation's own grid values (rows of root and weight,
-// 46 KB, which stay in L1) and weights them by the 5-point Lagrange basis, the
-// same interpolant as the power-form records (232 KB): 20 more FP64 operations
-// for L1 instead of L2 latency, (ps|ss) of 91 waters without digestion 37.7 ->
-// 34.6 ms.  N = 2, 3 (118, 206 KB of rows) gained nothing and keep the records.
 template <typename R, int N>
 __device__ __forceinline__ void rys_roots_all(R T, R* root, R* weight) {
     if (T >= R(c_tabs.tmax[N])) {
@@ -204,12 +199,21 @@ __device__ __forceinline__ void rys_roots_all(R T, R* root, R* weight) {
         return;
     }
     using V2 = typename RysTab<R>::V2;
+    // floor by adding 1.5 x 2^52 (2^23) to fi - 1/2: the grid index is the low
+    // word, without the conversions' quarter-rate pipe.  On a grid point the
+    // rounding may pick the record before it with t = 1, the same value.
     const R fi = T * R(100);
-    const int k = static_cast<int>(fi);
-    const R t = fi - R(k);
-    constexpr bool RAW = sizeof(R) == 8 && N == 1;
-    const V2* rec = RAW ? reinterpret_cast<const V2*>(c_tabs.rys_raw1) + k
-                        : reinterpret_cast<const V2*>(RysTab<R>::h(N)) + k * (5 * N);
+    int k;
+    R t;
+    if constexpr (sizeof(R) == 8) {
+        const R m = (fi - R(0.5)) + R(6755399441055744.0);
+        k = __double2loint(m);
+        t = fi - (m - R(6755399441055744.0));
+    } else {
+        k = static_cast<int>(fi);
+        t = fi - R(k);
+    }
+    const V2* rec = reinterpret_cast<const V2*>(RysTab<R>::h(N)) + k * (5 * N);
     R c[5][2 * N];
 #pragma unroll
     for (int j = 0; j < 5; ++j)
@@ -219,29 +223,14 @@ __device__ __forceinline__ void rys_roots_all(R T, R* root, R* weight) {
             c[j][2 * m] = v.x;
             c[j][2 * m + 1] = v.y;
         }
-    if constexpr (RAW) {
-        const R u = t - R(2), s = u * u, A = s - R(1), B = s - R(4);
-        const R ua = (u * R(1.0 / 24.0)) * A, ub = (u * R(-1.0 / 6.0)) * B, ua2 = ua + ua;
-        const R l0 = ua * u - ua2, l1 = ub * u - ub, l2 = (R(0.25) * A) * B, l3 = ub * u + ub, l4 = ua * u + ua2;
 #pragma unroll
-        for (int i = 0; i < 2 * N; ++i) {
-            R v = c[4][i] * l4;
-            v = v + c[0][i] * l0;
-            v = v + c[3][i] * l3;
-            v = v + c[1][i] * l1;
-            v = v + c[2][i] * l2;
-            if (i < N) root[i] = v; else weight[i - N] = v;
-        }
-    } else {
-#pragma unroll
-        for (int i = 0; i < 2 * N; ++i) {
-            R v = c[4][i];
-            v = v * t + c[3][i];
-            v = v * t + c[2][i];
-            v = v * t + c[1][i];
-            v = v * t + c[0][i];
-            if (i < N) root[i] = v; else weight[i - N] = v;
-        }
+    for (int i = 0; i < 2 * N; ++i) {
+        R v = c[4][i];
+        v = v * t + c[3][i];
+        v = v * t + c[2][i];
+        v = v * t + c[1][i];
+        v = v * t + c[0][i];
+        if (i < N) root[i] = v; else weight[i - N] = v;
     }
 }
 
@@ -255,9 +244,11 @@ __device__ __forceinline__ void rys_roots_smem32(float T, const float* __restric
         rys_asymptotic<float, N>(T, root, weight);
         return;
     }
-    const float x = T * float(kRys32PerUnitDev);
-    const int k = static_cast<int>(x);
-    const float u = x - float(k) - 0.5f;
+    // floor as in rys_roots_all; u = x - k - 1/2
+    const float x = T * float(kRys32PerUnitDev) - 0.5f;
+    const float m = x + 12582912.0f;
+    const int k = __float_as_int(m) - 0x4B400000;
+    const float u = x - (m - 12582912.0f);
     const float2* rec = reinterpret_cast<const float2*>(table + k * (kRys32CoefDev * 2 * N));
     float c[kRys32CoefDev][2 * N];
 #pragma unroll

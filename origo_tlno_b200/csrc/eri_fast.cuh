@@ -127,10 +127,13 @@ struct FastShape {
     // classes whose carried sums are small.
     static constexpr int GB = (TPQ == 1 && NSA * (NSC + NSD) + NSCD <= kMaxCarried) ? kBraGroup : 1;
     static constexpr int LANE_STRIDE = (NAS * NSCD) | 1;  // odd: conflict-free FP64 rows
-    static constexpr int SMEM_DOUBLES = TPQ == 1 ? 0 : BBQ * 32 * LANE_STRIDE;
+    static constexpr int SMEM_VALS = TPQ == 1 ? 0 : BBQ * 32 * LANE_STRIDE;  // in the kernel's precision
     // Bra-group classes: per lane, the density values every bra of a block
     // shares (D[a,c], D[a,d], D[c,d]), gathered once per tile.
     static constexpr int PRE_VALS = GB > 1 ? NSA * NSC + NSA * NSD + NSCD : 0;
+    // Density values of one quartet that no other bra shares: D[b,c], D[b,d] of
+    // a bra-group class, all of D[a,c], D[a,d], D[b,c], D[b,d], D[c,d] else.
+    static constexpr int OWN_VALS = GB > 1 ? NSB * (NSC + NSD) : (NSA + NSB) * (NSC + NSD) + NSCD;
 };
 
 // Binomial C(n, k) for the small HRR exponents.
@@ -206,10 +209,35 @@ __device__ __forceinline__ T pair_transfer(const T* X, Src&& src) {
     return out;
 }
 
+// Ket side of a lane's quartet.
 struct QuartetGeom {
-    double A[3], C[3];
-    double AB[3], CD[3];
+    double C[3], CD[3];
+    int ok, npk;  // primitive records
+    const PairRec* rec;
 };
+
+// Separation, shells and first functions of a pair, read again where the
+// transfer and the digestion need them: held in registers across the primitive
+// loop they cost the ungrouped classes spills.
+__device__ __forceinline__ void reload_ab(const PairRec* p, double* ab) {
+#pragma unroll
+    for (int k = 0; k < 3; ++k)
+        asm volatile("ld.global.f64 %0, [%1];" : "=d"(ab[k]) : "l"(&p->AB[k]));
+}
+__device__ __forceinline__ void reload_ids(const PairRec* p, int& shA, int& shB, int& a0, int& b0) {
+    asm volatile("ld.global.v2.s32 {%0, %1}, [%2];" : "=r"(shA), "=r"(shB) : "l"(&p->shA));
+    asm volatile("ld.global.v2.s32 {%0, %1}, [%2];" : "=r"(a0), "=r"(b0) : "l"(&p->a0));
+}
+
+// Asynchronous copy of one density element into this lane's shared slot.
+template <typename R>
+__device__ __forceinline__ void async_copy(R* dst, const R* src) {
+    asm volatile("cp.async.ca.shared.global [%0], [%1], %2;" ::"r"(static_cast<unsigned>(__cvta_generic_to_shared(dst))),
+                 "l"(src), "n"(sizeof(R))
+                 : "memory");
+}
+__device__ __forceinline__ void async_commit() { asm volatile("cp.async.commit_group;" ::: "memory"); }
+__device__ __forceinline__ void async_wait() { asm volatile("cp.async.wait_group 0;" ::: "memory"); }
 
 // This lane's share of a quartet's primitive loops: ket primitives ik0,
 // ik0 + ikn, ..., bra primitives ib0, ib0 + ibn, ...; `lanes` lanes (a power
@@ -220,7 +248,7 @@ struct LaneSplit {
 
 // Phase 1 + 2 for slice G (rows ia = G, G+TPQ, ...).
 template <typename R, int LA, int LB, int LC, int LD, int G>
-__device__ __forceinline__ void fast_slice(const PlanView& pv, int bra, int ket, bool active, const QuartetGeom& q,
+__device__ __forceinline__ void fast_slice(const PlanView& pv, const PairRec& br, const QuartetGeom& q, bool active,
                                            const LaneSplit& sp, double fs_thr2, const float* rtab,
                                            R* __restrict__ ks) {
     using S = FastShape<LA, LB, LC, LD>;
@@ -232,8 +260,8 @@ __device__ __forceinline__ void fast_slice(const PlanView& pv, int bra, int ket,
         for (int ic = 0; ic < S::NCS; ++ic) acc[rr][ic] = R(0);
 
     if (active) {
-        const int npb = __ldg(pv.pair_nprim + bra), npk = __ldg(pv.pair_nprim + ket);
-        const int ob = __ldg(pv.pair_prim_off + bra), ok = __ldg(pv.pair_prim_off + ket);
+        const int npb = br.nprim, npk = q.npk;
+        const int ob = br.prim_off, ok = q.ok;
         // FP64: 48-byte records {p, Px, Py, Pz, w, 1/p} read as three 16-byte
         // vectors.  FP32: 24-byte records {p, P-A, w, 1/p} relative to the
         // pair's first centre, PQ = (P-A) - (Q-C) + (A-C).
@@ -242,14 +270,14 @@ __device__ __forceinline__ void fast_slice(const PlanView& pv, int bra, int ket,
         const float2* pb32 = reinterpret_cast<const float2*>(pv.prim32 + ob);
         const float2* pk32 = reinterpret_cast<const float2*>(pv.prim32 + ok);
         constexpr bool F32 = std::is_same<R, float>::value;
-        const R ACx = R(q.A[0] - q.C[0]), ACy = R(q.A[1] - q.C[1]), ACz = R(q.A[2] - q.C[2]);
-        // Primitive FASTSCHWARZ: a primitive quartet whose estimate product is
-        // below the squared threshold contributes nothing (per lane; the
-        // reference drops a SIMD packet only when every lane fails).
-        const bool fs_on = fs_thr2 > 0.0;
+        const R ACx = R(br.A[0] - q.C[0]), ACy = R(br.A[1] - q.C[1]), ACz = R(br.A[2] - q.C[2]);
         // Ket primitive outer, bra primitive inner: each lane gathers its own
         // ket record once per bra, and the bra records (the same for every
         // lane of the warp) are broadcast loads.
+        // Primitive FASTSCHWARZ (FS): a primitive quartet whose estimate
+        // product is below the squared threshold contributes nothing (per
+        // lane; the reference drops a SIMD packet only when every lane fails).
+        auto prim_loop = [&](auto fs_on) {
         for (int ik = sp.ik0; ik < npk; ik += sp.ikn) {
             const double fsk = fs_on ? __ldg(pv.prim_fs + ok + ik) : 0.0;
             R qe, QCx, QCy, QCz, kw, kip;
@@ -275,7 +303,7 @@ __device__ __forceinline__ void fast_slice(const PlanView& pv, int bra, int ket,
                     const double2 b0v = __ldg(pb + 3 * ib), b1v = __ldg(pb + 3 * ib + 1), b2v = __ldg(pb + 3 * ib + 2);
                     const double bp_x = b0v.y, bp_y = b1v.x, bp_z = b1v.y;
                     p = R(b0v.x);
-                    PAx = R(bp_x - q.A[0]); PAy = R(bp_y - q.A[1]); PAz = R(bp_z - q.A[2]);
+                    PAx = R(bp_x - br.A[0]); PAy = R(bp_y - br.A[1]); PAz = R(bp_z - br.A[2]);
                     bw = R(b2v.x); bip = R(b2v.y);
                     PQx = R(bp_x - kp_x); PQy = R(bp_y - kp_y); PQz = R(bp_z - kp_z);
                 }
@@ -347,6 +375,17 @@ __device__ __forceinline__ void fast_slice(const PlanView& pv, int bra, int ket,
                 }
             }
         }
+        };
+        // Two copies of the loop, so that the unscreened one carries no test:
+        // FP32 light classes of 91 waters 67.8 -> 62.6 ms, FP64 110 -> 107 ms.
+        // A sliced class keeps one copy per slice, and FP64 with two or more roots
+        // spills with two.
+        if constexpr (S::TPQ == 1 && (F32 || S::N == 1)) {
+            if (fs_thr2 > 0.0) prim_loop(std::true_type{});
+            else prim_loop(std::false_type{});
+        } else {
+            prim_loop(fs_thr2 > 0.0);
+        }
     }
 
     // Sum of a split quartet's lanes (the split is the same for the whole warp).
@@ -359,7 +398,16 @@ __device__ __forceinline__ void fast_slice(const PlanView& pv, int bra, int ket,
 
     // Phase 2: ket transfer + projection of the owned rows (in R: the FP32
     // kernels keep the whole quartet in FP32 up to the FP64 atomics).
-    const R CDr[3] = {R(q.CD[0]), R(q.CD[1]), R(q.CD[2])};
+    R CDr[3] = {R(0), R(0), R(0)};
+    if constexpr (S::GB > 1) {
+#pragma unroll
+        for (int k = 0; k < 3; ++k) CDr[k] = R(q.CD[k]);
+    } else if constexpr (LD > 0) {
+        double cd[3];
+        reload_ab(q.rec, cd);
+#pragma unroll
+        for (int k = 0; k < 3; ++k) CDr[k] = R(cd[k]);
+    }
     sfor<ROWS>([&](auto RR) {
         constexpr int rr = TLNO_CI(RR);
         constexpr int ia = G + rr * S::TPQ;
@@ -374,15 +422,15 @@ __device__ __forceinline__ void fast_slice(const PlanView& pv, int bra, int ket,
 }
 
 template <typename R, int LA, int LB, int LC, int LD, int G = 0>
-__device__ __forceinline__ void fast_slice_dispatch(int g, const PlanView& pv, int bra, int ket, bool active,
-                                                    const QuartetGeom& q, const LaneSplit& sp, double fs_thr2,
-                                                    const float* rtab, R* ks) {
+__device__ __forceinline__ void fast_slice_dispatch(int g, const PlanView& pv, const PairRec& br,
+                                                    const QuartetGeom& q, bool active, const LaneSplit& sp,
+                                                    double fs_thr2, const float* rtab, R* ks) {
     using S = FastShape<LA, LB, LC, LD>;
     if constexpr (G < S::TPQ) {
         if (g == G)
-            fast_slice<R, LA, LB, LC, LD, G>(pv, bra, ket, active, q, sp, fs_thr2, rtab, ks);
+            fast_slice<R, LA, LB, LC, LD, G>(pv, br, q, active, sp, fs_thr2, rtab, ks);
         else
-            fast_slice_dispatch<R, LA, LB, LC, LD, G + 1>(g, pv, bra, ket, active, q, sp, fs_thr2, rtab, ks);
+            fast_slice_dispatch<R, LA, LB, LC, LD, G + 1>(g, pv, br, q, active, sp, fs_thr2, rtab, ks);
     }
 }
 
@@ -401,29 +449,35 @@ __device__ __forceinline__ bool group_any(bool pred, int id, int nthreads) {
     return r != 0;
 }
 
-// The lightest classes (at most 9 radial accumulators per thread) are
-// latency-bound on their gathers: a register cap of 4 resident CTAs per SM
-// (FP64) or 6 (FP32) buys more warps than it costs (measured on 200 waters);
-// classes with larger accumulator blocks would spill under it.  FP32 (ps|ss)
-// takes 7 (cfg4: 1199 -> 1119 ms; 7 or 8 is slower or equal on the other
-// light classes).
+// Resident CTAs per SM (the register cap).  The lightest classes (at most 9
+// radial accumulators per thread) wait on their gathers, so a cap buys warps
+// until it spills into the primitive loop; per class on 91 waters, ms at
+// 3 | 4 | 5 CTAs in FP64 and 4 | 5 | 6 in FP32:
+//   (ss|ss) 19.9 | 19.9 | 17.9   12.8 | 11.9 | 11.6
+//   (ps|ss) 50.4 | 44.4 | 52.1   28.8 | 26.8 | 30.0
+//   (ps|ps) 35.4 | 33.6 | 42.5   20.3 | 25.1 | 27.2
+//   (pp|ss) 20.9 | 19.3 | 21.6   12.6 | 13.7 | 14.3
+//   (ds|ss) 11.6 | 10.4 | 12.3    6.6 |  7.4 |  8.0
+// Unsliced FP32 classes with larger accumulator blocks: 3 resident CTAs instead
+// of the 2 their ~200 registers allow, 4 for (pp|ps), (ds|ps), (dp|ss),
+// (ds|ds), (dd|ss).
 template <typename R, int LA, int LB, int LC, int LD>
 __host__ __device__ constexpr int fast_min_blocks() {
     using S = FastShape<LA, LB, LC, LD>;
-    // unsliced FP32 classes with larger accumulator blocks: 3 resident CTAs
-    // instead of the 2 their ~200 registers allow, 4 for (pp|ps), (ds|ps),
-    // (dp|ss), (ds|ds), (dd|ss) (measured per class on 200 waters; 4 is
-    // slower on the others)
-    if (S::TPQ == 1 && S::NAS * S::NCS > 9) {
-        if (!std::is_same<R, float>::value) return 1;
+    constexpr bool F32 = std::is_same<R, float>::value;
+    if (S::TPQ > 1) return 1;
+    if (S::NAS * S::NCS > 9) {
+        // FP64 (dp|ss) 9.1 -> 7.5 ms with 3; the others lose to spills
+        if (!F32) return LA == 2 && LB == 1 && LC == 0 ? 3 : 1;
         constexpr bool four = (LA == 1 && LB == 1 && LC == 1 && LD == 0) || (LA == 2 && LB == 0 && LC == 1 && LD == 0) ||
                               (LA == 2 && LB == 1 && LC == 0 && LD == 0) || (LA == 2 && LB == 0 && LC == 2 && LD == 0) ||
                               (LA == 2 && LB == 2 && LC == 0 && LD == 0);
         return four ? 4 : 3;
     }
-    if (!(S::TPQ == 1 && S::NAS * S::NCS <= 9)) return 1;
-    if (!std::is_same<R, float>::value) return 4;
-    return (LA == 1 && LB == 0 && LC == 0 && LD == 0) ? 7 : 6;
+    if (LA == 0) return F32 ? 6 : 5;                        // (ss|ss)
+    if (LA == 1 && LB == 0 && LC == 0) return F32 ? 5 : 4;  // (ps|ss)
+    if (LA == 1 && LB == 0) return 4;             // (ps|ps)
+    return 4;
 }
 
 // Where a bra-group class keeps the per-tile density values of a lane:
@@ -437,6 +491,52 @@ __host__ __device__ constexpr int fast_pre_mode() {
     if (S::PRE_VALS == 0) return 0;
     if (std::is_same<R, double>::value) return 2;
     return fast_min_blocks<R, LA, LB, LC, LD>() > 1 ? 2 : 1;
+}
+
+// Whether the sums carried across a block's bras live in shared memory: FP64
+// (ps|ps), whose 15 sums then leave room for 4 resident CTAs without spills
+// (91 waters 35.4 -> 33.6 ms, without digestion 25.2 -> 21.3 ms).  (ss|ss),
+// (ps|ss), (pp|ss), (ds|ss) lose 0-4%: theirs fit the registers.
+template <typename R, int LA, int LB, int LC, int LD>
+__host__ __device__ constexpr bool fast_carry_smem() {
+    using S = FastShape<LA, LB, LC, LD>;
+    return std::is_same<R, double>::value && LA == 1 && LB == 0 && LC == 1;
+}
+
+// Whether a quartet's own density values are copied asynchronously to shared
+// memory while its primitives are evaluated.  Gathered at their use they were
+// one L2 latency after the other at 8 to 16 resident warps.  Ungrouped classes,
+// with | without, ms on 91 waters: FP64 (dp|pp) 20.9 | 22.6, (dp|dp) 7.5 | 7.6,
+// FP32 (dp|pp) 14.5 | 16.8, (ds|pp) 9.9 | 12.8 (with the 64-bit addresses
+// before).  FP64 ungrouped classes spill, and the slots take L1 from the spills:
+// (dp|ds) 1.02 | 0.88, (fp|pp) 3.80 | 2.80, (fs|pp) 0.52 | 0.50 (f-shell 14
+// atoms), so not above 48 KB per CTA nor with an f bra; and nowhere at the cost
+// of a resident CTA.
+template <typename R, int LA, int LB, int LC, int LD>
+__host__ __device__ constexpr bool fast_async() {
+    using S = FastShape<LA, LB, LC, LD>;
+    constexpr bool F32 = std::is_same<R, float>::value;
+    if (S::GB > 1) return true;
+    constexpr int kSmem = 220 * 1024;
+    const int own = S::BBQ * 32 * (S::OWN_VALS + 2) * static_cast<int>(sizeof(R));
+    if (!F32 && (LA > 2 || own > 48 * 1024)) return false;
+    const int base = S::SMEM_VALS * static_cast<int>(sizeof(R)) + (F32 && S::N <= 3 ? 26 * 1024 : 1024);
+    const int regs = S::WARPS > 4 ? 1 : fast_min_blocks<R, LA, LB, LC, LD>() > 2 ? fast_min_blocks<R, LA, LB, LC, LD>() : 2;
+    const int before = kSmem / base < regs ? kSmem / base : regs;
+    return kSmem / (base + own) >= before;
+}
+
+// Shared memory of one warp group's region (see the kernel), a multiple of 16
+// bytes.
+template <typename R, int LA, int LB, int LC, int LD>
+__host__ __device__ constexpr int fast_region_bytes() {
+    using S = FastShape<LA, LB, LC, LD>;
+    if (!fast_async<R, LA, LB, LC, LD>()) return 0;
+    const int pre = fast_pre_mode<R, LA, LB, LC, LD>() == 2 ? S::PRE_VALS : 0;
+    const int car = fast_carry_smem<R, LA, LB, LC, LD>() ? S::PRE_VALS : 0;
+    const int bytes = (S::GB > 1 ? S::GB * (static_cast<int>(sizeof(PairRec)) + 4) : 0) +
+                      (S::GB * S::NSAB + 32 * (S::OWN_VALS + pre + car)) * static_cast<int>(sizeof(R));
+    return (bytes + 15) / 16 * 16;
 }
 
 template <typename R, int LA, int LB, int LC, int LD>
@@ -459,9 +559,9 @@ __global__ void __launch_bounds__(32 * FastShape<LA, LB, LC, LD>::WARPS, fast_mi
     // FP32 kernels with N <= 3 stage their Rys interval polynomials in shared
     // memory behind the row-exchange buffer.
     const float* rtab = nullptr;
-    int smem_used = S::SMEM_DOUBLES * 8;  // bytes
+    int smem_used = S::SMEM_VALS * static_cast<int>(sizeof(R));  // bytes (a multiple of 128)
     if constexpr (std::is_same<R, float>::value && S::N <= 3) {
-        float* t = reinterpret_cast<float*>(fast_smem + S::SMEM_DOUBLES);
+        float* t = reinterpret_cast<float*>(reinterpret_cast<unsigned char*>(fast_smem) + smem_used);
         const int n4 = c_tabs.rys32_nint[S::N] * (kRys32CoefDev * 2 * S::N) / 4;
         const float4* src = reinterpret_cast<const float4*>(c_tabs.rys32[S::N]);
         for (int i = threadIdx.x; i < n4; i += blockDim.x) reinterpret_cast<float4*>(t)[i] = __ldg(src + i);
@@ -469,10 +569,23 @@ __global__ void __launch_bounds__(32 * FastShape<LA, LB, LC, LD>::WARPS, fast_mi
         rtab = t;
         smem_used += n4 * 16;
     }
-    // this warp's slots of the per-tile density values (shared-memory mode)
+    // The warp group's region: (bra-group classes) the pair records of the
+    // block's bras; D[a,b] of the bras; the asynchronous density values of a
+    // quartet; (bra-group classes) the per-tile density values.
     constexpr int PRE_MODE = fast_pre_mode<R, LA, LB, LC, LD>();
-    R* pre = reinterpret_cast<R*>(reinterpret_cast<unsigned char*>(fast_smem) + smem_used) +
-             (PRE_MODE == 2 ? warp * 32 * S::PRE_VALS : 0);
+    constexpr bool GROUP = S::GB > 1;
+    constexpr bool ASYNC = fast_async<R, LA, LB, LC, LD>();
+    unsigned char* wsm = reinterpret_cast<unsigned char*>(fast_smem) + smem_used +
+                         grp * fast_region_bytes<R, LA, LB, LC, LD>();
+    PairRec* wrec = reinterpret_cast<PairRec*>(wsm);
+    int* wbra = reinterpret_cast<int*>(wsm + S::GB * sizeof(PairRec));
+    R* wdab = reinterpret_cast<R*>(wsm + (GROUP ? S::GB * (sizeof(PairRec) + sizeof(int)) : 0));
+    R* dg = wdab + S::GB * S::NSAB;
+    R* pre = dg + S::OWN_VALS * 32;
+    R* carry = pre + (PRE_MODE == 2 ? S::PRE_VALS * 32 : 0);
+    int staged = -1;               // block whose bras are staged
+    double qmax = 0.0, qmin = 0.0; // bounds of the staged bras
+    int imax = 0;                  // largest class index of the staged bras
     __shared__ int s_chunk[S::BBQ];
     const int ntiles = cl.tile_end - cl.tile_begin;
     double csum = 0.0;  // ERI checksum stream: this thread's share
@@ -517,112 +630,134 @@ __global__ void __launch_bounds__(32 * FastShape<LA, LB, LC, LD>::WARPS, fast_mi
         const bool lane_ok = j < bd.nket;
         const int ket = bd.ket0 + (lane_ok ? j : 0);
 
-        // Quick test on the Schwarz products alone: a tile without any quartet
-        // for this launch (bound, triangle, precision pass) is left before
-        // the ket geometry is loaded.
-        const double qket = __ldg(pv.pair_Q + ket);
         const int mol = pv.pair_mol ? __ldg(pv.pair_mol + ket) : 0;
+        const int M = pv.mol_M ? __ldg(pv.mol_M + mol) : cl.M;
+        const long long mbase = pv.mol_mat_off ? __ldg(pv.mol_mat_off + mol) : 0;
+        // Element (r, c) of the molecule's matrices: M <= 65535, so the index
+        // fits 32 bits.  FP32 kernels gather from the FP32 copy of the density.
+        auto at = [&](int r, int c) { return static_cast<unsigned>(r) * static_cast<unsigned>(M) + static_cast<unsigned>(c); };
+        // k: constant column offset, kept out of the 32-bit index so that the
+        // elements of a row share one address
+        auto dp = [&](int r, int c, int k) -> const R* {
+            if constexpr (std::is_same<R, float>::value) return cl.dens32 + mbase + at(r, c) + k;
+            else return cl.dens + mbase + at(r, c) + k;
+        };
+        auto dm = [&](int r, int c, int k) { return __ldg(dp(r, c, k)); };
+        auto add_j = [&](int r, int c, int k, R v) { atomicAdd(cl.J + mbase + at(r, c) + k, double(v)); };
+        auto add_k = [&](int r, int c, int k, R v) { atomicAdd(cl.K + mbase + at(r, c) + k, double(v)); };
         // the density screen raises the Schwarz cutoff of this build
         const double tau_t = cl.den.mode ? density_tau_min(cl, mol) : cl.tau;
-        {
-            bool act = false;
-            for (int ib = 0; ib < S::GB && ib < bd.nbra; ++ib) {
-                const int bra = __ldg(cl.bra_list + bd.bra0 + ib);
-                if (!lane_ok || (cl.same && bd.koff + j > bra - bd.xbeg)) continue;
-                const double qq = __ldg(pv.pair_Q + bra) * qket;
-                bool a = qq >= tau_t;
-                if (cl.prec_mode == 1) a = a && qq >= thr;
-                if (cl.prec_mode == 2) a = a && !(qq >= thr);
-                act = act || a;
+
+        if constexpr (GROUP) {
+            // Pair records and D[a,b] of the block's bras, once per block: the
+            // bra loop then reads shared memory instead of walking list ->
+            // pair -> shell -> density.
+            if (b != staged) {
+                staged = b;
+                __syncwarp();
+                for (int x = lane; x < bd.nbra * 5; x += 32) {
+                    const int w = x / 5;
+                    const int bra = __ldg(cl.bra_list + bd.bra0 + w);
+                    reinterpret_cast<int4*>(wrec + w)[x - 5 * w] =
+                        __ldg(reinterpret_cast<const int4*>(pv.pair_rec + bra) + (x - 5 * w));
+                    if (x == 5 * w) wbra[w] = bra;
+                }
+                __syncwarp();
+                if (cl.want_j)
+                    for (int x = lane; x < bd.nbra * S::NSAB; x += 32) {
+                        const int w = x / S::NSAB, e = x - w * S::NSAB;
+                        wdab[x] = dm(wrec[w].a0 + e / S::NSB, wrec[w].b0, e % S::NSB);
+                    }
+                qmax = qmin = wrec[0].Q;
+                imax = wbra[0] - bd.xbeg;
+                for (int w = 1; w < bd.nbra; ++w) {
+                    qmax = fmax(qmax, wrec[w].Q);
+                    qmin = fmin(qmin, wrec[w].Q);
+                    imax = max(imax, wbra[w] - bd.xbeg);
+                }
+                __syncwarp();
             }
-            bool any_tile;
-            if constexpr (S::TPQ > 1)
-                any_tile = group_any(act, bar_id, bar_n);
-            else
-                any_tile = __any_sync(0xffffffffu, act);
-            if (!any_tile) continue;
         }
 
         // ket side, once per tile
-        const int C = __ldg(pv.pair_A + ket), D = __ldg(pv.pair_B + ket);
+        const PairRec kr = load_pair_rec(pv.pair_rec + ket);
+        const double qket = kr.Q;
+        if constexpr (GROUP) {
+            // A tile without any quartet for this launch (bound, triangle,
+            // precision pass) is left before its density values are loaded.
+            bool act = lane_ok && !(cl.same && bd.koff + j > imax) && qmax * qket >= tau_t;
+            if (cl.prec_mode == 1) act = act && qmax * qket >= thr;
+            if (cl.prec_mode == 2) act = act && !(qmin * qket >= thr);
+            if (!__any_sync(0xffffffffu, act)) continue;
+        }
+        int C = kr.shA, D = kr.shB, c0 = kr.a0, d0 = kr.b0;
         QuartetGeom q;
 #pragma unroll
         for (int k = 0; k < 3; ++k) {
-            q.C[k] = __ldg(pv.shell_xyz + 3 * C + k);
-            q.CD[k] = q.C[k] - __ldg(pv.shell_xyz + 3 * D + k);
+            q.C[k] = kr.A[k];
+            q.CD[k] = kr.AB[k];
         }
-        const int M = pv.mol_M ? __ldg(pv.mol_M + mol) : cl.M;
-        const long long mbase = pv.mol_mat_off ? __ldg(pv.mol_mat_off + mol) : 0;
-        const double* Dm = cl.dens + mbase;
-        double* Jm = cl.J + mbase;
-        double* Km = cl.K + mbase;
-        // FP32 kernels gather from the FP32 copy of the density
-        const float* Dm32 = cl.dens32 + mbase;
-        auto dm = [&](int r, int c) {
-            if constexpr (std::is_same<R, float>::value)
-                return R(__ldg(Dm32 + (long long)r * M + c));
-            else
-                return __ldg(Dm + (long long)r * M + c);
-        };
-        const int c0 = __ldg(pv.shell_sph + C), d0 = __ldg(pv.shell_sph + D);
+        q.rec = pv.pair_rec + ket;
+        q.ok = kr.prim_off;
+        q.npk = kr.nprim;
 
         // Sums carried across the bras of a block (they share the first
         // shell A): J[cd], K[ac], K[ad] of this lane's ket.
         constexpr bool CARRY = S::GB > 1;
-        R jcd[CARRY ? S::NSCD : 1];
-        R kacc[CARRY ? S::NSA : 1][CARRY ? S::NSC : 1];
-        R kadc[CARRY ? S::NSA : 1][CARRY ? S::NSD : 1];
+        // in the order of the per-tile density values: K[ac], K[ad], J[cd].
+        constexpr bool CAR_SMEM = fast_carry_smem<R, LA, LB, LC, LD>();
+        R creg[CARRY && !CAR_SMEM ? S::PRE_VALS : 1];
+        auto car = [&](int k) -> R& {
+            if constexpr (CAR_SMEM) return carry[k * 32 + lane];
+            else return creg[k];
+        };
         if constexpr (CARRY) {
 #pragma unroll
-            for (int t = 0; t < S::NSCD; ++t) jcd[t] = 0.0;
-#pragma unroll
-            for (int a = 0; a < S::NSA; ++a) {
-#pragma unroll
-                for (int c = 0; c < S::NSC; ++c) kacc[a][c] = 0.0;
-#pragma unroll
-                for (int d = 0; d < S::NSD; ++d) kadc[a][d] = 0.0;
-            }
+            for (int k = 0; k < S::PRE_VALS; ++k) car(k) = R(0);
         }
         // The bras of a block share shell A, so the lane's D[a, c], D[a, d]
         // and D[c, d] are the same for every bra of it: they are gathered once
         // per tile, into registers or this lane's shared-memory slots
         // [k * 32 + lane].
-        constexpr bool PRE = PRE_MODE != 0;
         R preg[PRE_MODE == 1 ? S::PRE_VALS : 1];
         auto pre_at = [&](int k) -> R& {
             if constexpr (PRE_MODE == 1) return preg[k];
             else return pre[k * 32 + lane];
         };
-        if constexpr (PRE) {
-            const int a0b = __ldg(pv.shell_sph + __ldg(pv.pair_A + __ldg(cl.bra_list + bd.bra0)));
+        if constexpr (PRE_MODE != 0) {
+            const int a0b = wrec[0].a0;
             if (cl.want_k) {
 #pragma unroll
                 for (int sa = 0; sa < S::NSA; ++sa) {
 #pragma unroll
-                    for (int sc = 0; sc < S::NSC; ++sc) pre_at(sa * S::NSC + sc) = dm(a0b + sa, c0 + sc);
+                    for (int sc = 0; sc < S::NSC; ++sc) pre_at(sa * S::NSC + sc) = dm(a0b + sa, c0, sc);
 #pragma unroll
                     for (int sd = 0; sd < S::NSD; ++sd)
-                        pre_at(S::NSA * S::NSC + sa * S::NSD + sd) = dm(a0b + sa, d0 + sd);
+                        pre_at(S::NSA * S::NSC + sa * S::NSD + sd) = dm(a0b + sa, d0, sd);
                 }
             }
             if (cl.want_j) {
 #pragma unroll
                 for (int t = 0; t < S::NSCD; ++t)
-                    pre_at(S::NSA * (S::NSC + S::NSD) + t) = dm(c0 + t / S::NSD, d0 + t % S::NSD);
+                    pre_at(S::NSA * (S::NSC + S::NSD) + t) = dm(c0 + t / S::NSD, d0, t % S::NSD);
             }
         }
         bool touched = false;
         int a0 = 0;
 
         for (int ib = 0; ib < S::GB && ib < bd.nbra; ++ib) {
-            const int bra = __ldg(cl.bra_list + bd.bra0 + ib);
+            // GB == 1: the record of the block's bra, the same for every lane
+            PairRec one;
+            if constexpr (!GROUP) one = load_pair_rec(pv.pair_rec + __ldg(cl.bra_list + bd.bra0));
+            const PairRec& br = GROUP ? wrec[ib] : one;
+            const int bra = GROUP ? wbra[ib] : __ldg(cl.bra_list + bd.bra0);
             const int i = bra - bd.xbeg;
-            const int A = __ldg(pv.pair_A + bra), B = __ldg(pv.pair_B + bra);
+            int A = br.shA, B = br.shB;
             bool active = lane_ok && !(cl.same && bd.koff + j > i);
             // density screen: Coulomb and exchange contributions kept apart
             R jon = R(1), kon = R(1);
             if (active) {
-                const double qq = __ldg(pv.pair_Q + bra) * qket;
+                const double qq = br.Q * qket;
                 active = qq >= cl.tau;
                 if (cl.prec_mode == 1) active = active && qq >= thr;
                 if (cl.prec_mode == 2) active = active && !(qq >= thr);
@@ -641,26 +776,101 @@ __global__ void __launch_bounds__(32 * FastShape<LA, LB, LC, LD>::WARPS, fast_mi
                 any = __any_sync(0xffffffffu, active);
             if (!any) continue;
             touched = touched || (active && digester);
-
+            a0 = br.a0;
+            int b0 = br.b0;
+            // the quartet's density values, in flight during the primitive loop;
+            // the warps of a sliced quartet share the copies
+            constexpr int BX = GROUP ? 0 : S::NSA * (S::NSC + S::NSD);  // first D[b,c] slot of a lane
+            constexpr int CX = BX + S::NSB * (S::NSC + S::NSD);         // first D[c,d] slot
+            if constexpr (ASYNC) {
+                auto copy = [&](int k, int r, int c, int off) {
+                    if (S::TPQ == 1 || k % S::TPQ == g) async_copy(dg + k * 32 + lane, dp(r, c, off));
+                };
+                if (cl.want_k && active && digester) {
 #pragma unroll
-            for (int k = 0; k < 3; ++k) {
-                q.A[k] = __ldg(pv.shell_xyz + 3 * A + k);
-                q.AB[k] = q.A[k] - __ldg(pv.shell_xyz + 3 * B + k);
+                    for (int sb = 0; sb < S::NSB; ++sb) {
+#pragma unroll
+                        for (int sc = 0; sc < S::NSC; ++sc) copy(BX + sb * S::NSC + sc, b0 + sb, c0, sc);
+#pragma unroll
+                        for (int sd = 0; sd < S::NSD; ++sd)
+                            copy(BX + S::NSB * S::NSC + sb * S::NSD + sd, b0 + sb, d0, sd);
+                    }
+                    if constexpr (!GROUP) {
+#pragma unroll
+                        for (int sa = 0; sa < S::NSA; ++sa) {
+#pragma unroll
+                            for (int sc = 0; sc < S::NSC; ++sc) copy(sa * S::NSC + sc, a0 + sa, c0, sc);
+#pragma unroll
+                            for (int sd = 0; sd < S::NSD; ++sd)
+                                copy(S::NSA * S::NSC + sa * S::NSD + sd, a0 + sa, d0, sd);
+                        }
+                    }
+                }
+                if constexpr (!GROUP) {
+                    if (cl.want_j && active && digester) {
+#pragma unroll
+                        for (int t = 0; t < S::NSCD; ++t) copy(CX + t, c0 + t / S::NSD, d0, t % S::NSD);
+                    }
+                    if (cl.want_j && g == 0)
+                        for (int e = lane; e < S::NSAB; e += 32) async_copy(wdab + e, dp(a0 + e / S::NSB, b0, e % S::NSB));
+                }
+                async_commit();
             }
-            fast_slice_dispatch<R, LA, LB, LC, LD>(g, pv, bra, ket, active, q, sp, cl.fs_thr2, rtab, ks);
+            auto d_ac = [&](int sa, int sc) -> R {
+                if constexpr (PRE_MODE != 0) return pre_at(sa * S::NSC + sc);
+                else if constexpr (ASYNC) return dg[(sa * S::NSC + sc) * 32 + lane];
+                else return dm(a0 + sa, c0, sc);
+            };
+            auto d_ad = [&](int sa, int sd) -> R {
+                if constexpr (PRE_MODE != 0) return pre_at(S::NSA * S::NSC + sa * S::NSD + sd);
+                else if constexpr (ASYNC) return dg[(S::NSA * S::NSC + sa * S::NSD + sd) * 32 + lane];
+                else return dm(a0 + sa, d0, sd);
+            };
+            auto d_bc = [&](int sb, int sc) -> R {
+                if constexpr (ASYNC) return dg[(BX + sb * S::NSC + sc) * 32 + lane];
+                else return dm(b0 + sb, c0, sc);
+            };
+            auto d_bd = [&](int sb, int sd) -> R {
+                if constexpr (ASYNC) return dg[(BX + S::NSB * S::NSC + sb * S::NSD + sd) * 32 + lane];
+                else return dm(b0 + sb, d0, sd);
+            };
+            auto d_cd = [&](int sc, int sd) -> R {
+                const int t = sc * S::NSD + sd;
+                if constexpr (PRE_MODE != 0) return pre_at(S::NSA * (S::NSC + S::NSD) + t);
+                else if constexpr (ASYNC) return dg[(CX + t) * 32 + lane];
+                else return dm(c0 + sc, d0, sd);
+            };
+            auto d_ab = [&](int ib_, int e) -> R {
+                if constexpr (ASYNC) return wdab[ib_ * S::NSAB + e];
+                else return dm(a0 + e / S::NSB, b0, e % S::NSB);
+            };
+            fast_slice_dispatch<R, LA, LB, LC, LD>(g, pv, br, q, active, sp, cl.fs_thr2, rtab, ks);
             // one lane of a split quartet digests it
             active = active && digester;
+            if constexpr (!GROUP) {
+                reload_ids(pv.pair_rec + bra, A, B, a0, b0);
+                reload_ids(q.rec, C, D, c0, d0);
+            }
+            if constexpr (ASYNC) async_wait();
             if constexpr (S::TPQ > 1) group_sync(bar_id, bar_n);
+            else if constexpr (ASYNC && !GROUP) __syncwarp();
 
             // ---- bra transfer + projection per owned ket column, digestion ----
-            a0 = __ldg(pv.shell_sph + A);
-            const int b0 = __ldg(pv.shell_sph + B);
             R f = active ? R(1) : R(0);
             if (A == B) f *= R(0.5);
             if (C == D) f *= R(0.5);
             if (bra == ket) f *= R(0.5);
             const R fj = R(4) * f * jon, fk = R(2) * f * kon;
-            const R ABr[3] = {R(q.AB[0]), R(q.AB[1]), R(q.AB[2])};
+            R ABr[3] = {R(0), R(0), R(0)};
+            if constexpr (GROUP) {
+#pragma unroll
+                for (int k = 0; k < 3; ++k) ABr[k] = R(br.AB[k]);
+            } else if constexpr (LB > 0) {
+                double ab[3];
+                reload_ab(pv.pair_rec + bra, ab);
+#pragma unroll
+                for (int k = 0; k < 3; ++k) ABr[k] = R(ab[k]);
+            }
 
             R jab[S::NSAB];
 #pragma unroll
@@ -712,14 +922,12 @@ __global__ void __launch_bounds__(32 * FastShape<LA, LB, LC, LD>::WARPS, fast_mi
                         if (cl.want_j) {
                             R s = R(0);
 #pragma unroll
-                            for (int e = 0; e < S::NSAB; ++e) s += V[e] * R(dm(a0 + e / S::NSB, b0 + e % S::NSB));
+                            for (int e = 0; e < S::NSAB; ++e) s += V[e] * d_ab(ib, e);
                             if constexpr (CARRY)
-                                jcd[t] += fj * s;
+                                car(S::NSA * (S::NSC + S::NSD) + t) += fj * s;
                             else
-                                atomicAdd(Jm + (long long)(c0 + sc) * M + d0 + sd, double(fj * s));
-                            R dcd;
-                            if constexpr (PRE) dcd = pre_at(S::NSA * (S::NSC + S::NSD) + t);
-                            else dcd = R(dm(c0 + sc, d0 + sd));
+                                add_j(c0 + sc, d0, sd, fj * s);
+                            const R dcd = d_cd(sc, sd);
 #pragma unroll
                             for (int e = 0; e < S::NSAB; ++e) jab[e] += V[e] * dcd;
                         }
@@ -728,19 +936,12 @@ __global__ void __launch_bounds__(32 * FastShape<LA, LB, LC, LD>::WARPS, fast_mi
                             R dbd[S::NSB], dbc[S::NSB];
 #pragma unroll
                             for (int sb = 0; sb < S::NSB; ++sb) {
-                                dbd[sb] = R(dm(b0 + sb, d0 + sd));
-                                dbc[sb] = R(dm(b0 + sb, c0 + sc));
+                                dbd[sb] = d_bd(sb, sd);
+                                dbc[sb] = d_bc(sb, sc);
                             }
 #pragma unroll
                             for (int sa = 0; sa < S::NSA; ++sa) {
-                                R dad, dac;
-                                if constexpr (PRE) {
-                                    dad = pre_at(S::NSA * S::NSC + sa * S::NSD + sd);
-                                    dac = pre_at(sa * S::NSC + sc);
-                                } else {
-                                    dad = R(dm(a0 + sa, d0 + sd));
-                                    dac = R(dm(a0 + sa, c0 + sc));
-                                }
+                                const R dad = d_ad(sa, sd), dac = d_ac(sa, sc);
                                 R sac = R(0), sad = R(0);
 #pragma unroll
                                 for (int sb = 0; sb < S::NSB; ++sb) {
@@ -751,8 +952,8 @@ __global__ void __launch_bounds__(32 * FastShape<LA, LB, LC, LD>::WARPS, fast_mi
                                     kbd[sb][sd] += v * dac;
                                 }
                                 if constexpr (CARRY) {
-                                    kacc[sa][sc] += fk * sac;
-                                    kadc[sa][sd] += fk * sad;
+                                    car(sa * S::NSC + sc) += fk * sac;
+                                    car(S::NSA * S::NSC + sa * S::NSD + sd) += fk * sad;
                                 } else {
                                     kac[sa] += sac;
                                     kad[sa][sd] += sad;
@@ -764,11 +965,11 @@ __global__ void __launch_bounds__(32 * FastShape<LA, LB, LC, LD>::WARPS, fast_mi
                         if constexpr (!CARRY) {
 #pragma unroll
                             for (int sa = 0; sa < S::NSA; ++sa)
-                                atomicAdd(Km + (long long)(a0 + sa) * M + c0 + sc, double(fk * kac[sa]));
+                                add_k(a0 + sa, c0, sc, fk * kac[sa]);
                         }
 #pragma unroll
                         for (int sb = 0; sb < S::NSB; ++sb)
-                            atomicAdd(Km + (long long)(b0 + sb) * M + c0 + sc, double(fk * kbc[sb]));
+                            add_k(b0 + sb, c0, sc, fk * kbc[sb]);
                     }
                 });
                 if (cl.want_k) {
@@ -782,11 +983,11 @@ __global__ void __launch_bounds__(32 * FastShape<LA, LB, LC, LD>::WARPS, fast_mi
                         if constexpr (!CARRY) {
 #pragma unroll
                             for (int sa = 0; sa < S::NSA; ++sa)
-                                atomicAdd(Km + (long long)(a0 + sa) * M + d0 + sd, double(fk * kad[sa][sd]));
+                                add_k(a0 + sa, d0, sd, fk * kad[sa][sd]);
                         }
 #pragma unroll
                         for (int sb = 0; sb < S::NSB; ++sb)
-                            atomicAdd(Km + (long long)(b0 + sb) * M + d0 + sd, double(fk * kbd[sb][sd]));
+                            add_k(b0 + sb, d0, sd, fk * kbd[sb][sd]);
                     });
                 }
             }
@@ -797,7 +998,7 @@ __global__ void __launch_bounds__(32 * FastShape<LA, LB, LC, LD>::WARPS, fast_mi
                     R s = fj * jab[e];
 #pragma unroll
                     for (int o = 16; o > 0; o >>= 1) s += __shfl_xor_sync(0xffffffffu, s, o);
-                    if (lane == 0 && s != R(0)) atomicAdd(Jm + (long long)(a0 + e / S::NSB) * M + b0 + e % S::NSB, double(s));
+                    if (lane == 0 && s != R(0)) add_j(a0 + e / S::NSB, b0, e % S::NSB, s);
                 }
             }
             if constexpr (S::TPQ > 1) group_sync(bar_id, bar_n);
@@ -809,15 +1010,15 @@ __global__ void __launch_bounds__(32 * FastShape<LA, LB, LC, LD>::WARPS, fast_mi
                 if (cl.want_j) {
 #pragma unroll
                     for (int t = 0; t < S::NSCD; ++t)
-                        atomicAdd(Jm + (long long)(c0 + t / S::NSD) * M + d0 + t % S::NSD, double(jcd[t]));
+                        add_j(c0 + t / S::NSD, d0, t % S::NSD, car(S::NSA * (S::NSC + S::NSD) + t));
                 }
                 if (cl.want_k) {
 #pragma unroll
                     for (int sa = 0; sa < S::NSA; ++sa) {
 #pragma unroll
-                        for (int sc = 0; sc < S::NSC; ++sc) atomicAdd(Km + (long long)(a0 + sa) * M + c0 + sc, double(kacc[sa][sc]));
+                        for (int sc = 0; sc < S::NSC; ++sc) add_k(a0 + sa, c0, sc, car(sa * S::NSC + sc));
 #pragma unroll
-                        for (int sd = 0; sd < S::NSD; ++sd) atomicAdd(Km + (long long)(a0 + sa) * M + d0 + sd, double(kadc[sa][sd]));
+                        for (int sd = 0; sd < S::NSD; ++sd) add_k(a0 + sa, d0, sd, car(S::NSA * S::NSC + sa * S::NSD + sd));
                     }
                 }
             }
@@ -839,14 +1040,13 @@ constexpr int fast_bras() { return FastShape<LA, LB, LC, LD>::GB; }
 template <int LA, int LB, int LC, int LD>
 constexpr int fast_groups() { return FastShape<LA, LB, LC, LD>::BBQ; }
 template <int LA, int LB, int LC, int LD>
-constexpr int fast_smem_bytes() { return FastShape<LA, LB, LC, LD>::SMEM_DOUBLES * 8; }
+constexpr int fast_smem_bytes(bool fp32) { return FastShape<LA, LB, LC, LD>::SMEM_VALS * (fp32 ? 4 : 8); }
 template <int LA, int LB, int LC, int LD>
 constexpr int fast_roots() { return FastShape<LA, LB, LC, LD>::N; }
 template <int LA, int LB, int LC, int LD>
-constexpr int fast_pre_bytes(bool fp32) {
+constexpr int fast_group_bytes(bool fp32) {
     using S = FastShape<LA, LB, LC, LD>;
-    return fp32 ? (fast_pre_mode<float, LA, LB, LC, LD>() == 2 ? S::WARPS * 32 * S::PRE_VALS * 4 : 0)
-                : (fast_pre_mode<double, LA, LB, LC, LD>() == 2 ? S::WARPS * 32 * S::PRE_VALS * 8 : 0);
+    return S::BBQ * (fp32 ? fast_region_bytes<float, LA, LB, LC, LD>() : fast_region_bytes<double, LA, LB, LC, LD>());
 }
 
 }  // namespace dev

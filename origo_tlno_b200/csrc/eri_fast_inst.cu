@@ -16,14 +16,14 @@
 namespace tlno_gpu {
 
 // Dynamic shared memory: the row-exchange buffer of a sliced class, the FP32
-// Rys interval polynomials in the FP32 kernels with N <= 3, and the per-tile
-// density slots of the bra-group classes.
+// Rys interval polynomials in the FP32 kernels with N <= 3, and the
+// bra-group regions.
 #define TLNO_FAST_IMPL(id, a, b, c, d)                                                                  \
     static int fast_smem_##id(bool fp32) {                                                              \
         constexpr int n = dev::fast_roots<a, b, c, d>();                                                \
-        int bytes = dev::fast_smem_bytes<a, b, c, d>();                                                 \
+        int bytes = dev::fast_smem_bytes<a, b, c, d>(fp32);                                             \
         if (fp32 && n <= kRys32MaxN) bytes += rys32_intervals(n) * (kRys32Deg + 1) * 2 * n * 4;         \
-        bytes += dev::fast_pre_bytes<a, b, c, d>(fp32);                                                 \
+        bytes += dev::fast_group_bytes<a, b, c, d>(fp32);                                               \
         return bytes;                                                                                   \
     }                                                                                                   \
     void fast_upload_##id(const dev::DevTables& t, const dev::CartTable& ct, const dev::C2STable& cs) {  \

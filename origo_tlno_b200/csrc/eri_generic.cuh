@@ -473,14 +473,12 @@ template <typename R>
 __device__ void generic_quartet_cta(const PlanView& pv, const ClassLaunch& cl, const GenericCtaLayout& lay,
                                     double* sm, int bra, int ket, bool jon, bool kon) {
     const int tid = threadIdx.x, nt = blockDim.x;
-    const int A = pv.pair_A[bra], B = pv.pair_B[bra];
-    const int C = pv.pair_A[ket], D = pv.pair_B[ket];
-    const double* xa = pv.shell_xyz + 3 * A;
-    const double* xc = pv.shell_xyz + 3 * C;
+    const PairRec br = load_pair_rec(pv.pair_rec + bra), kr = load_pair_rec(pv.pair_rec + ket);
+    const double *xa = br.A, *xc = kr.A;
     const int la = cl.la, lb = cl.lb, lc = cl.lc, ld = cl.ld;
     const int nroots = (la + lb + lc + ld) / 2 + 1;
-    const int npb = pv.pair_nprim[bra], npk = pv.pair_nprim[ket];
-    const int pob = pv.pair_prim_off[bra], pok = pv.pair_prim_off[ket];
+    const int npb = br.nprim, npk = kr.nprim;
+    const int pob = br.prim_off, pok = kr.prim_off;
     const DPrimPair* pb = pv.prim + pob;
     const DPrimPair* pk = pv.prim + pok;
     R* Gs = reinterpret_cast<R*>(sm);
@@ -570,92 +568,7 @@ __device__ void generic_quartet_cta(const PlanView& pv, const ClassLaunch& cl, c
     }
     __syncthreads();
 
-    if (cl.checksum) {
-        // ERI checksum stream: canonical unique elements of the block
-        const int a0 = pv.shell_sph[A], b0 = pv.shell_sph[B];
-        const int c0 = pv.shell_sph[C], d0 = pv.shell_sph[D];
-        double s = 0.0;
-        for (int e = tid; e < lay.nsab * lay.nscd; e += nt) {
-            const int sab = e / lay.nscd, scd = e - sab * lay.nscd;
-            if (canonical_element(A == B, C == D, bra == ket, a0, sab / lay.nb, b0, sab % lay.nb, c0,
-                                  scd / lay.nd, d0, scd % lay.nd))
-                s += V[e];
-        }
-        for (int o = 16; o > 0; o >>= 1) s += __shfl_xor_sync(0xffffffffu, s, o);
-        if ((tid & 31) == 0 && s != 0.0) atomicAdd(cl.checksum, s);
-        __syncthreads();
-        return;
-    }
-    // J/K digestion with shell-level degeneracy f (consumer_policies.ipp:87-157)
-    const int mol = pv.pair_mol ? pv.pair_mol[bra] : 0;
-    const int M = pv.mol_M ? pv.mol_M[mol] : cl.M;
-    const long long mbase = pv.mol_mat_off ? pv.mol_mat_off[mol] : 0;
-    const double* Dm = cl.dens + mbase;
-    double* Jm = cl.J + mbase;
-    double* Km = cl.K + mbase;
-    const int a0 = pv.shell_sph[A], b0 = pv.shell_sph[B];
-    const int c0 = pv.shell_sph[C], d0 = pv.shell_sph[D];
-    double f = 1.0;
-    if (A == B) f *= 0.5;
-    if (C == D) f *= 0.5;
-    if (bra == ket) f *= 0.5;
-    const int na = lay.na, nb = lay.nb, nc = lay.nc, nd = lay.nd;
-    double* Pab = sm + lay.off_P;
-    double* Pcd = Pab + na * nb;
-    double* Pbd = Pcd + nc * nd;
-    double* Pbc = Pbd + nb * nd;
-    double* Pad = Pbc + nb * nc;
-    double* Pac = Pad + na * nd;
-    for (int e = tid; e < na * nb; e += nt) Pab[e] = Dm[(long long)(a0 + e / nb) * M + b0 + e % nb];
-    for (int e = tid; e < nc * nd; e += nt) Pcd[e] = Dm[(long long)(c0 + e / nd) * M + d0 + e % nd];
-    for (int e = tid; e < nb * nd; e += nt) Pbd[e] = Dm[(long long)(b0 + e / nd) * M + d0 + e % nd];
-    for (int e = tid; e < nb * nc; e += nt) Pbc[e] = Dm[(long long)(b0 + e / nc) * M + c0 + e % nc];
-    for (int e = tid; e < na * nd; e += nt) Pad[e] = Dm[(long long)(a0 + e / nd) * M + d0 + e % nd];
-    for (int e = tid; e < na * nc; e += nt) Pac[e] = Dm[(long long)(a0 + e / nc) * M + c0 + e % nc];
-    __syncthreads();
-    const int nscd = lay.nscd;
-    if (cl.want_j && jon) {
-        const double fj = 4.0 * f;
-        for (int sab = tid; sab < na * nb; sab += nt) {
-            double s = 0.0;
-            for (int t = 0; t < nscd; ++t) s += V[sab * nscd + t] * Pcd[t];
-            atomicAdd(Jm + (long long)(a0 + sab / nb) * M + b0 + sab % nb, fj * s);
-        }
-        for (int scd = tid; scd < nscd; scd += nt) {
-            double s = 0.0;
-            for (int t = 0; t < na * nb; ++t) s += V[t * nscd + scd] * Pab[t];
-            atomicAdd(Jm + (long long)(c0 + scd / nd) * M + d0 + scd % nd, fj * s);
-        }
-    }
-    if (cl.want_k && kon) {
-        const double fk = 2.0 * f;
-        const int nac = na * nc, nad = na * nd, nbc = nb * nc, nbd = nb * nd;
-        for (int e = tid; e < nac + nad + nbc + nbd; e += nt) {
-            double s = 0.0;
-            if (e < nac) {
-                const int a = e / nc, c = e % nc;
-                for (int b = 0; b < nb; ++b)
-                    for (int d = 0; d < nd; ++d) s += V[(a * nb + b) * nscd + c * nd + d] * Pbd[b * nd + d];
-                atomicAdd(Km + (long long)(a0 + a) * M + c0 + c, fk * s);
-            } else if (e < nac + nad) {
-                const int k = e - nac, a = k / nd, d = k % nd;
-                for (int b = 0; b < nb; ++b)
-                    for (int c = 0; c < nc; ++c) s += V[(a * nb + b) * nscd + c * nd + d] * Pbc[b * nc + c];
-                atomicAdd(Km + (long long)(a0 + a) * M + d0 + d, fk * s);
-            } else if (e < nac + nad + nbc) {
-                const int k = e - nac - nad, b = k / nc, c = k % nc;
-                for (int a = 0; a < na; ++a)
-                    for (int d = 0; d < nd; ++d) s += V[(a * nb + b) * nscd + c * nd + d] * Pad[a * nd + d];
-                atomicAdd(Km + (long long)(b0 + b) * M + c0 + c, fk * s);
-            } else {
-                const int k = e - nac - nad - nbc, b = k / nd, d = k % nd;
-                for (int a = 0; a < na; ++a)
-                    for (int c = 0; c < nc; ++c) s += V[(a * nb + b) * nscd + c * nd + d] * Pac[a * nc + c];
-                atomicAdd(Km + (long long)(b0 + b) * M + d0 + d, fk * s);
-            }
-        }
-    }
-    __syncthreads();
+    block_digest(pv, cl, lay, sm, V, br, kr, bra, ket, jon, kon);
 }
 
 // Tiled schedule (J/K mode), one quartet per block at a time: tile = 1 bra

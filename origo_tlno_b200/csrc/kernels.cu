@@ -361,6 +361,24 @@ __global__ void fma_peak_kernel(R* out, int iters, R seed) {
     if (s == R(-12345)) out[0] = s;  // keeps the chains live
 }
 
+__global__ void pair_records_kernel(PlanView pv, int n, PairRec* out) {
+    for (int k = blockIdx.x * blockDim.x + threadIdx.x; k < n; k += gridDim.x * blockDim.x) {
+        PairRec r;
+        r.Q = pv.pair_Q[k];
+        r.shA = pv.pair_A[k];
+        r.shB = pv.pair_B[k];
+        for (int x = 0; x < 3; ++x) {
+            r.A[x] = pv.shell_xyz[3 * r.shA + x];
+            r.AB[x] = r.A[x] - pv.shell_xyz[3 * r.shB + x];
+        }
+        r.a0 = pv.shell_sph[r.shA];
+        r.b0 = pv.shell_sph[r.shB];
+        r.prim_off = pv.pair_prim_off[k];
+        r.nprim = pv.pair_nprim[k];
+        out[k] = r;
+    }
+}
+
 // Power-form records of the 5-point Newton-forward interpolant on rows
 // k..k+4 of the Rys table: with forward differences d1 = D f0,
 // d2 = D^2 f0 / 2, d3 = D^3 f0 / 6, d4 = D^4 f0 / 24,
@@ -415,14 +433,6 @@ void ensure_device_tables() {
         const std::vector<double> rec = rys_power_records(h, n);
         t.rys_h[n] = upload(rec);
         t.rys_h32[n] = upload(std::vector<float>(rec.begin(), rec.end()));
-        if (n == 1) {
-            std::vector<double> rows;
-            for (int r = 0; r < h.rys_rows[1]; ++r) {
-                rows.push_back(h.rys_roots[1][r]);
-                rows.push_back(h.rys_weights[1][r]);
-            }
-            t.rys_raw1 = upload(rows);
-        }
         t.tmax[n] = h.rys_tmax[n];
         for (int i = 0; i < n; ++i) {
             t.h2[n][i] = h.herm_root2[n][i];
@@ -497,6 +507,13 @@ void launch_pair_projectors(const int* pair_A, const int* pair_B, const double* 
     TLNO_CUDA(cudaGetLastError());
 }
 
+void launch_pair_records(const PlanView& pv, int n_pairs, PairRec* out, cudaStream_t s) {
+    if (n_pairs == 0) return;
+    const int grid = std::min((n_pairs + 255) / 256, sm_count() * 8);
+    pair_records_kernel<<<grid, 256, 0, s>>>(pv, n_pairs, out);
+    TLNO_CUDA(cudaGetLastError());
+}
+
 // CTA shape of the generic J/K kernel for a class: threads per block and item
 // slots per batch, and the dynamic shared memory it needs.
 static void generic_cta_shape(int la, int lb, int lc, int ld, int& threads, int& nb_items, int& bytes) {
@@ -527,10 +544,7 @@ void launch_eri_jk_generic(const PlanView& pv, const ClassLaunch& cl, bool fp32,
         }
         const long long ntiles = cl.tile_end - cl.tile_begin;
         const int wave = sm_count() * std::max(per_sm, 1);
-        // kets per fetch: a whole tile where every block fetches at least 16
-        // times, halved down to one quartet where the schedule is smaller
-        int part = cl.bk;
-        while (part > 1 && ntiles * ((cl.bk + part - 1) / part) < 16LL * wave) part = (part + 1) / 2;
+        const int part = block_tile_part(ntiles, cl.bk, wave);
         const int g = static_cast<int>(std::max(1LL, std::min<long long>(ntiles * ((cl.bk + part - 1) / part), wave)));
         if (fp32)
             eri_generic_cta_jk_kernel<float><<<g, threads, bytes, s>>>(pv, cl, nb_items, part);

@@ -9,6 +9,7 @@ namespace dev {
 struct PlanView;
 struct ClassLaunch;
 struct OneeLaunch;
+struct PairRec;
 }  // namespace dev
 
 // Uploads the constant tables (Boys, Rys, Cartesian, cart->sph) for the
@@ -29,6 +30,19 @@ void launch_eri_jk_generic(const dev::PlanView& pv, const dev::ClassLaunch& cl, 
 // when the class has no specialised kernel.
 bool launch_eri_jk_fast(const dev::PlanView& pv, const dev::ClassLaunch& cl, bool fp32,
                         int grid, cudaStream_t s);
+// Largest dynamic shared memory of a block-per-quartet kernel (they hold a
+// little static shared memory too).
+constexpr int kMaxBlockSmem = 226 * 1024;
+// Kets per fetch of the block-per-quartet kernels: a whole tile where every
+// resident block fetches at least 16 times, halved down to one quartet where
+// the schedule is smaller.
+inline int block_tile_part(long long ntiles, int bk, int wave) {
+    int part = bk;
+    while (part > 1 && ntiles * ((bk + part - 1) / part) < 16LL * wave) part = (part + 1) / 2;
+    return part;
+}
+// Pair records of a plan (view with its pair and shell arrays filled).
+void launch_pair_records(const dev::PlanView& pv, int n_pairs, dev::PairRec* out, cudaStream_t s);
 bool has_fast_kernel(int la, int lb, int lc, int ld);
 // Bra pairs per CTA of the compile-time kernel of a class (its schedule's
 // block height).

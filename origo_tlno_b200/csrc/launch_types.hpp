@@ -15,6 +15,18 @@ struct FPrimPair {
     float p, PAx, PAy, PAz, w, invp;
 };
 
+// What the ERI kernels need of one shell pair, in one 80-byte record read as
+// five 16-byte vectors (bound, first centre, separation, shells, first
+// spherical functions, primitive records).
+struct alignas(16) PairRec {
+    double Q;
+    double A[3];
+    double AB[3];
+    int shA, shB;
+    int a0, b0;
+    int prim_off, nprim;
+};
+
 // Device view of one plan (or of a batch of plans: every pair carries the
 // AO offset of its molecule, so one launch can serve many molecules).
 struct PlanView {
@@ -26,6 +38,7 @@ struct PlanView {
     const int* pair_prim_off;
     const int* pair_nprim;
     const double* pair_Q;         // Schwarz bound
+    const PairRec* pair_rec;      // the pair arrays above as records (J/K plans; else null)
     const int* pair_mol;          // molecule of the pair (batch), may be null
     const DPrimPair* prim;
     const FPrimPair* prim32;      // same records in FP32 (P relative to A), may be null

@@ -381,6 +381,7 @@ dev::PlanView Plan2e::view() const {
     pv.pair_prim_off = d_pair_prim_off.as<int>();
     pv.pair_nprim = d_pair_nprim.as<int>();
     pv.pair_Q = d_pair_Q.as<double>();
+    pv.pair_rec = d_pair_rec.as<dev::PairRec>();
     pv.pair_mol = n_mol > 1 ? d_pair_mol.as<int>() : nullptr;
     pv.prim = d_prim.as<dev::DPrimPair>();
     pv.prim32 = d_prim32.as<dev::FPrimPair>();
@@ -476,6 +477,8 @@ void build_plan(Plan2e& plan, const std::vector<const Basis*>& bases, std::vecto
     upload_vec(plan.d_pair_prim_off, plan.pair_prim_off, s);
     upload_vec(plan.d_pair_Q, plan.pair_Q, s);
     upload_vec(plan.d_pair_mol, plan.pair_mol, s);
+    plan.d_pair_rec.alloc(sizeof(dev::PairRec) * std::max<std::size_t>(plan.pair_A.size(), 1));
+    launch_pair_records(plan.view(), static_cast<int>(plan.pair_A.size()), plan.d_pair_rec.as<dev::PairRec>(), s);
     upload_vec(plan.d_prim, prim, s);
     upload_vec(plan.d_prim32, prim32, s);
     upload_vec(plan.d_mol_mat_off, plan.mol_mat_off, s);
