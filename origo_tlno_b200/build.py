@@ -22,7 +22,7 @@ CUDA_HOME = os.environ.get("CUDA_HOME", "/usr/local/cuda")
 NVCC = os.path.join(CUDA_HOME, "bin", "nvcc")
 ARCH = ["-gencode", "arch=compute_100a,code=sm_100a"]
 
-CU_SOURCES = ["kernels.cu", "noalloc.cu"]
+CU_SOURCES = ["kernels.cu", "eri_rows.cu", "noalloc.cu"]
 def _fast_count():
     """Number of compile-time ERI classes (TLNO_FAST_COUNT in csrc/fast_classes.hpp)."""
     import re

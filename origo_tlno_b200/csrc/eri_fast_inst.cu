@@ -235,11 +235,6 @@ namespace tlno_gpu {
 #else
 #define TLNO_FAST_IF_34(x)
 #endif
-#if TLNO_FAST_ID == 35
-#define TLNO_FAST_IF_35(x) x
-#else
-#define TLNO_FAST_IF_35(x)
-#endif
 
 TLNO_FAST_CLASSES(TLNO_FAST_SELECT)
 

@@ -1,8 +1,13 @@
 // Classes with a compile-time ERI kernel (la >= lb, lc >= ld, bra class
-// index >= ket class index): every class with shells up to d and the f
-// classes with one f shell whose instantiation compiles in a few minutes
-// (bra (fs), (fp) against kets up to (dp)/(fs), (fd) against (ss), (ps),
-// (ds)).  The other f classes take the warp-per-quartet kernel.  Each class
+// index >= ket class index): every class with shells up to d except (dd|dd)
+// and the f classes with one f shell whose instantiation compiles in a few
+// minutes (bra (fs), (fp) against kets up to (dp)/(fs), (fd) against (ss),
+// (ps), (ds)).  The other classes take the block-per-quartet kernel
+// (eri_rows.cuh); (dd|dd), 8 slices of spilled registers here, runs there in
+// 0.53 instead of 1.01 ms (f-shell 14 atoms), 0.098 / 0.094 ms (24-atom
+// organic), 0.61 / 0.54 ms of 290 (91 waters).  (dd|dp), (fp|dp), (fp|pp) gain
+// there only with deep contractions (3.7 / 4.7, 4.0 / 4.7, 2.9 / 2.8 ms, but
+// 16.8 / 5.2 ms for (dd|dp) of 91 waters) and stay.  Each class
 // is compiled in its own translation unit (eri_fast_inst.cu with
 // -DTLNO_FAST_ID=<index>).
 #pragma once
@@ -30,24 +35,23 @@
     X(17, 2, 2, 1, 1) \
     X(18, 2, 2, 2, 0) \
     X(19, 2, 2, 2, 1) \
-    X(20, 2, 2, 2, 2) \
-    X(21, 3, 0, 0, 0) \
-    X(22, 3, 0, 1, 0) \
-    X(23, 3, 0, 1, 1) \
-    X(24, 3, 0, 2, 0) \
-    X(25, 3, 0, 2, 1) \
-    X(26, 3, 0, 2, 2) \
-    X(27, 3, 0, 3, 0) \
-    X(28, 3, 1, 0, 0) \
-    X(29, 3, 1, 1, 0) \
-    X(30, 3, 1, 1, 1) \
-    X(31, 3, 1, 2, 0) \
-    X(32, 3, 1, 2, 1) \
-    X(33, 3, 2, 0, 0) \
-    X(34, 3, 2, 1, 0) \
-    X(35, 3, 2, 2, 0)
+    X(20, 3, 0, 0, 0) \
+    X(21, 3, 0, 1, 0) \
+    X(22, 3, 0, 1, 1) \
+    X(23, 3, 0, 2, 0) \
+    X(24, 3, 0, 2, 1) \
+    X(25, 3, 0, 2, 2) \
+    X(26, 3, 0, 3, 0) \
+    X(27, 3, 1, 0, 0) \
+    X(28, 3, 1, 1, 0) \
+    X(29, 3, 1, 1, 1) \
+    X(30, 3, 1, 2, 0) \
+    X(31, 3, 1, 2, 1) \
+    X(32, 3, 2, 0, 0) \
+    X(33, 3, 2, 1, 0) \
+    X(34, 3, 2, 2, 0)
 
-#define TLNO_FAST_COUNT 36
+#define TLNO_FAST_COUNT 35
 
 namespace tlno_gpu {
 namespace dev {

@@ -454,6 +454,7 @@ void ensure_device_tables() {
 #define TLNO_FAST_UPLOAD(id, a, b, c, d) fast_upload_##id(t, ct, c2s);
     TLNO_FAST_CLASSES(TLNO_FAST_UPLOAD)
 #undef TLNO_FAST_UPLOAD
+    rows_upload(t, ct, c2s);
     TLNO_CUDA(cudaGetLastError());
     // The generic kernel may need more than 48 KB of dynamic shared memory.
     const int maxsm = 227 * 1024;
@@ -533,6 +534,7 @@ void launch_eri_jk_generic(const PlanView& pv, const ClassLaunch& cl, bool fp32,
                            cudaStream_t s) {
     if (cl.tile_end <= cl.tile_begin) return;
     if (pv.proj && warps <= 0) {
+        if (launch_eri_jk_rows(pv, cl, fp32, sm_count(), s)) return;
         // one quartet per block at a time, projectors from the plan
         int threads = 0, nb_items = 0, bytes = 0;
         generic_cta_shape(cl.la, cl.lb, cl.lc, cl.ld, threads, nb_items, bytes);

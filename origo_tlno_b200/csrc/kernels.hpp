@@ -10,6 +10,9 @@ struct PlanView;
 struct ClassLaunch;
 struct OneeLaunch;
 struct PairRec;
+struct DevTables;
+struct CartTable;
+struct C2STable;
 }  // namespace dev
 
 // Uploads the constant tables (Boys, Rys, Cartesian, cart->sph) for the
@@ -41,6 +44,10 @@ inline int block_tile_part(long long ntiles, int bk, int wave) {
     while (part > 1 && ntiles * ((bk + part - 1) / part) < 16LL * wave) part = (part + 1) / 2;
     return part;
 }
+// Block-per-quartet kernel of ket classes up to (ff) (eri_rows.cu); false for a
+// class it does not cover.
+void rows_upload(const dev::DevTables& t, const dev::CartTable& c, const dev::C2STable& s);
+bool launch_eri_jk_rows(const dev::PlanView& pv, const dev::ClassLaunch& cl, bool fp32, int sms, cudaStream_t s);
 // Pair records of a plan (view with its pair and shell arrays filled).
 void launch_pair_records(const dev::PlanView& pv, int n_pairs, dev::PairRec* out, cudaStream_t s);
 bool has_fast_kernel(int la, int lb, int lc, int ld);

@@ -1,8 +1,9 @@
-"""Tile shapes of the compile-time ERI kernels against the C++ restatement.
+"""Tile shapes of the ERI kernels against the C++ restatement.
 
 Small molecules make the schedule share a quartet's primitive loops between
 lanes and shorten the bra blocks; the primitive counts cover one, remainders
-of every lane count, and more bra than ket primitives.  FP64 sums of at most
+of every lane count, and more bra than ket primitives; two f shells of two
+primitives pass one item batch of the block-per-quartet kernel.  FP64 sums of at most
 a few thousand terms of magnitude <= 10 are exact to 1e-12.
 """
 import numpy as np
@@ -29,7 +30,8 @@ def _molecule(counts, seed):
 @pytest.mark.parametrize("counts", [
     [(0, 1), (1, 1)], [(0, 2), (1, 3)], [(0, 5), (1, 1), (2, 2)], [(0, 9), (1, 2), (2, 1)],
     [(0, 12), (1, 5)], [(0, 1), (1, 5), (2, 2)], [(0, 3), (2, 2), (3, 1)],
-], ids=lambda c: "-".join(f"{'spdf'[l]}{n}" for l, n in c))
+    [(1, 2), (2, 1), (3, 2)], [(1, 1), (4, 1)],
+], ids=lambda c: "-".join(f"{'spdfg'[l]}{n}" for l, n in c))
 def test_split_tiles_match_oracle(counts):
     if not port.available():
         pytest.skip("oracle not built")
