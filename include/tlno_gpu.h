@@ -317,7 +317,8 @@ void* tlno_gpu_batch_stream(tlno_gpu_batch* b);
  * capped by grid_mult x SMs), and streams (1..4): the class launches of a
  * build spread over that many streams (parallel branches of a captured
  * graph), so that the tail of one class overlaps the next; 1 keeps them in
- * order on the context's stream.  A per-class-combination generic override
+ * order on the context's stream.  Without this call a short build spreads
+ * over up to 8 streams and a long one keeps them in order.  A per-class-combination generic override
  * is set separately. */
 typedef struct {
     int generic_bk;

@@ -145,6 +145,24 @@ StreamFan::~StreamFan() {
     for (cudaEvent_t e : ev) cudaEventDestroy(e);
 }
 
+// Streams a build's launches spread over: as tuned, else up to 8 for a build
+// whose class launches are too short to fill the chip each (below
+// kFanMaxFlops), where their latencies overlap; a longer build runs them one
+// after the other, since neighbours then only share L2.  One stream | this
+// rule, ms: 2 waters (1.3e8 flops) 0.49 | 0.16, 17 atoms mixed (2.8e10) 3.00 |
+// 2.68; one | four streams: 40 waters (4.8e11) 44.4 | 46.0, f-shell 14 atoms
+// (3.6e11) 53.3 | 55.5, 160 waters (1.5e13) 1276 | 1307.
+namespace {
+constexpr double kFanMaxFlops = 1.5e11;
+// what a launch costs beside its flops, in flops (about 10 us of the chip)
+constexpr double kFanLaunchFlops = 1e8;
+int fan_streams(const Plan2e& plan, const Tuning& tune, std::size_t launches) {
+    if (tune.streams > 0) return std::min(tune.streams, 4);
+    if (plan.total_flops >= kFanMaxFlops) return 1;
+    return static_cast<int>(std::min<std::size_t>(8, std::max<std::size_t>(launches, 1)));
+}
+}  // namespace
+
 void enqueue_jk(Plan2e& plan, const Tuning& tune, const BuildSpec& spec, const double* dD, double* dJ,
                 double* dK, long long total, int M_single, double* d_dmax, float* dD32, cudaStream_t s,
                 StreamFan* fan) {
@@ -174,13 +192,25 @@ void enqueue_jk(Plan2e& plan, const Tuning& tune, const BuildSpec& spec, const d
     int sms = 0, devid = 0;
     TLNO_CUDA(cudaGetDevice(&devid));
     TLNO_CUDA(cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, devid));
-    // Class launches over `nst` streams: fork after the shared prologue
-    // (zeroing, max|D|, density tables), each class on the stream with the
-    // least flops so far (largest classes first), join before the
-    // symmetrisation.  J and K take FP64 atomics, so the order is free.
-    const int nst = (fan && tune.streams > 1) ? std::min(tune.streams, 4) : 1;
+    // The launches of the build: per class one, or (mixed build) the FP64 and
+    // the FP32 pass.  A class whose split multiplier is 0 stays FP64 in a mixed
+    // build (one launch, no FP32 pass).
+    struct Launch {
+        std::size_t ci;
+        int pass;
+    };
+    std::vector<Launch> launches;
+    for (std::size_t ci = 0; ci < plan.combos.size(); ++ci) {
+        const bool split = mixed && plan.combos[ci].mix_scale > 0.0;
+        for (int pass = 0; pass < (split ? 2 : 1); ++pass) launches.push_back({ci, pass});
+    }
+    // Launches over `nst` streams: fork after the shared prologue (zeroing,
+    // max|D|, density tables), each launch on the stream with the least flops
+    // so far (largest classes first), join before the symmetrisation.  J and K
+    // take FP64 atomics, so the order is free.
+    const int nst = fan ? fan_streams(plan, tune, launches.size()) : 1;
     std::vector<cudaStream_t> st(1, s);
-    std::vector<int> stream_of(plan.combos.size(), 0);
+    std::vector<int> stream_of(launches.size(), 0);
     if (nst > 1) {
         fan->ensure(nst - 1);
         TLNO_CUDA(cudaEventRecord(fan->ev[0], s));
@@ -188,20 +218,21 @@ void enqueue_jk(Plan2e& plan, const Tuning& tune, const BuildSpec& spec, const d
             TLNO_CUDA(cudaStreamWaitEvent(fan->aux[k], fan->ev[0], 0));
             st.push_back(fan->aux[k]);
         }
-        std::vector<std::size_t> order(plan.combos.size());
-        for (std::size_t i = 0; i < order.size(); ++i) order[i] = i;
-        std::stable_sort(order.begin(), order.end(),
-                         [&](std::size_t a, std::size_t b) { return plan.combos[a].flops > plan.combos[b].flops; });
+        std::stable_sort(launches.begin(), launches.end(), [&](const Launch& x, const Launch& y) {
+            return plan.combos[x.ci].flops > plan.combos[y.ci].flops;
+        });
         std::vector<double> load(nst, 0.0);
-        for (std::size_t i : order) {
+        for (std::size_t i = 0; i < launches.size(); ++i) {
             const int k = static_cast<int>(std::min_element(load.begin(), load.end()) - load.begin());
             stream_of[i] = k;
-            load[k] += plan.combos[i].flops;
+            load[k] += plan.combos[launches[i].ci].flops + kFanLaunchFlops;
         }
     }
-    for (std::size_t ci = 0; ci < plan.combos.size(); ++ci) {
+    for (std::size_t li = 0; li < launches.size(); ++li) {
+        const std::size_t ci = launches[li].ci;
+        const int pass = launches[li].pass;
         ComboSchedule& cs = plan.combos[ci];
-        cudaStream_t cs_stream = st[stream_of[ci]];
+        cudaStream_t cs_stream = st[stream_of[li]];
         dev::ClassLaunch cl{};
         cl.la = cs.la; cl.lb = cs.lb; cl.lc = cs.lc; cl.ld = cs.ld;
         cl.same = (cs.X == cs.Y);
@@ -228,20 +259,14 @@ void enqueue_jk(Plan2e& plan, const Tuning& tune, const BuildSpec& spec, const d
         cl.want_j = want_j;
         cl.want_k = want_k;
         const int grid = sms * tune.grid_mult;
-        // a class whose split multiplier is 0 stays FP64 in a mixed build
-        // (one launch, no FP32 pass)
         const bool split = mixed && cs.mix_scale > 0.0;
-        const int passes = split ? 2 : 1;
-        for (int pass = 0; pass < passes; ++pass) {
-            cl.prec_mode = split ? (pass + 1) : 0;
-            cl.counter = plan.d_counters.as<int>() + 2 * ci + pass;
-            const bool fp32 = split && pass == 1;
-            if (cs.fast) {
-                launch_eri_jk_fast(pv, cl, fp32, grid, cs_stream);
-            } else {
-                launch_eri_jk_generic(pv, cl, fp32, tune.generic_warps, grid, cs_stream);
-            }
-        }
+        cl.prec_mode = split ? (pass + 1) : 0;
+        cl.counter = plan.d_counters.as<int>() + 2 * ci + pass;
+        const bool fp32 = split && pass == 1;
+        if (cs.fast)
+            launch_eri_jk_fast(pv, cl, fp32, grid, cs_stream);
+        else
+            launch_eri_jk_generic(pv, cl, fp32, tune.generic_warps, grid, cs_stream);
     }
     if (nst > 1) {
         for (int k = 0; k < nst - 1; ++k) {

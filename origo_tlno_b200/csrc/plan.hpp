@@ -20,7 +20,7 @@ struct Tuning {
     int generic_bk = 64;    // ket pairs per tile of the warp-per-quartet kernel
     int generic_warps = 0;  // 0 = from shared-memory budget
     int grid_mult = 8;      // CTAs per SM for persistent launches
-    int streams = 1;        // streams the class launches of a build spread over
+    int streams = 0;        // streams the class launches of a build spread over (0 = by the plan's size)
     std::array<int, 256> force_generic{};  // per class combo: 1 = never use the fast kernel
 };
 
