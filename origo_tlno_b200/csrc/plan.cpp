@@ -66,6 +66,30 @@ void parallel_for(long long n, const std::function<void(long long, long long)>& 
     for (auto& t : ts) t.join();
 }
 
+// Runs f(t) on nt threads, t = 0 on this one; the first exception is rethrown
+// here.  Work is to be shared by an index of f's own: fewer threads may start.
+void run_threads(std::size_t nt, const std::function<void(std::size_t)>& f) {
+    std::mutex mtx;
+    std::exception_ptr failed;
+    auto guarded = [&](std::size_t t) {
+        try {
+            f(t);
+        } catch (...) {
+            std::lock_guard<std::mutex> lock(mtx);
+            if (!failed) failed = std::current_exception();
+        }
+    };
+    std::vector<std::thread> threads;
+    try {
+        for (std::size_t t = 1; t < nt; ++t) threads.emplace_back(guarded, t);
+    } catch (...) {
+    }
+    guarded(0);
+    for (auto& t : threads) t.join();
+    if (failed) std::rethrow_exception(failed);
+}
+std::size_t host_threads() { return std::max(1u, std::min(16u, std::thread::hardware_concurrency())); }
+
 inline void oriented(const Basis& b, int i, int j, int& A, int& B) {
     A = i;
     B = j;
@@ -724,31 +748,11 @@ void build_plan(Plan2e& plan, const std::vector<const Basis*>& bases, std::vecto
         cs.flops = fprim * cs.prim_quartets + fcon * cs.quartets;
     };
     {
-        // one class at a time per thread (the first exception is rethrown
-        // here); small plans are not worth a thread
+        // one class at a time per thread; small plans are not worth a thread
         std::atomic<std::size_t> next{0};
-        std::mutex mtx;
-        std::exception_ptr failed;
-        auto work = [&] {
-            try {
-                for (std::size_t k; (k = next.fetch_add(1)) < todo.size();) build_schedule(todo[k], resident[k]);
-            } catch (...) {
-                std::lock_guard<std::mutex> lock(mtx);
-                if (!failed) failed = std::current_exception();
-            }
-        };
-        const std::size_t nt = plan.kept_pairs < 2000
-                                   ? 1
-                                   : std::min<std::size_t>({std::max(1u, std::thread::hardware_concurrency()), 16,
-                                                            todo.size()});
-        std::vector<std::thread> threads;
-        try {
-            for (std::size_t t = 1; t < nt; ++t) threads.emplace_back(work);
-        } catch (...) {  // no more threads: the ones that started and this one do the work
-        }
-        work();
-        for (auto& t : threads) t.join();
-        if (failed) std::rethrow_exception(failed);
+        run_threads(plan.kept_pairs < 2000 ? 1 : std::min(host_threads(), todo.size()), [&](std::size_t) {
+            for (std::size_t k; (k = next.fetch_add(1)) < todo.size();) build_schedule(todo[k], resident[k]);
+        });
     }
     for (ComboSchedule& cs : todo) {
         if (cs.n_tiles == 0) continue;
@@ -842,41 +846,58 @@ void build_onee_plan(OneePlan& p, const Basis& b, double decay_eps, double nucle
         const Shell& s = b.shells[si];
         for (int i = 0; i < s.nprim; ++i) p.maxc[s.prim_offset + i] = gmax[b.onee_group[si]][i];
     }
-    for (int i = 0; i < ns; ++i) {
-        for (int j = 0; j <= i; ++j) {
-            const int gi = b.onee_group[i], gj = b.onee_group[j];
-            const Shell& si_ = b.shells[i];
-            const Shell& sj_ = b.shells[j];
-            const double dx = si_.center[0] - sj_.center[0], dy = si_.center[1] - sj_.center[1],
-                         dz = si_.center[2] - sj_.center[2];
-            const double r2 = dx * dx + dy * dy + dz * dz;
-            bool keep = true;
-            double bound = 0.0;
-            if (decay_eps > 0.0) {
-                const double mu = amin[gi] * amin[gj] / (amin[gi] + amin[gj]);
-                if (Kd[gi] * Kd[gj] * std::exp(-mu * r2) < decay_eps) keep = false;
-                if (keep) {
-                    const Shell& ri = b.shells[b.onee_group_rep[gi]];
-                    const Shell& rj = b.shells[b.onee_group_rep[gj]];
-                    for (int a = 0; a < ri.nprim; ++a)
-                        for (int c = 0; c < rj.nprim; ++c) {
-                            const double ea = b.exps[ri.prim_offset + a], ec = b.exps[rj.prim_offset + c];
-                            const double pp = ea + ec, chi = ea * ec / pp;
-                            bound += std::fabs(c_first(ri, a) * c_first(rj, c)) * std::pow(kPi / pp, 1.5) *
-                                     std::exp(-chi * r2);
-                        }
+    // Pair list, rows of shells dealt to host threads in blocks and joined in
+    // order.
+    constexpr int kRows = 16;
+    std::vector<std::vector<dev::OneePair>> part((ns + kRows - 1) / kRows);
+    auto rows = [&](int i0, std::vector<dev::OneePair>& out) {
+        for (int i = i0; i < std::min(ns, i0 + kRows); ++i) {
+            for (int j = 0; j <= i; ++j) {
+                const int gi = b.onee_group[i], gj = b.onee_group[j];
+                const Shell& si_ = b.shells[i];
+                const Shell& sj_ = b.shells[j];
+                const double dx = si_.center[0] - sj_.center[0], dy = si_.center[1] - sj_.center[1],
+                             dz = si_.center[2] - sj_.center[2];
+                const double r2 = dx * dx + dy * dy + dz * dz;
+                bool keep = true;
+                double bound = 0.0;
+                if (decay_eps > 0.0) {
+                    const double mu = amin[gi] * amin[gj] / (amin[gi] + amin[gj]);
+                    if (Kd[gi] * Kd[gj] * std::exp(-mu * r2) < decay_eps) keep = false;
+                    if (keep) {
+                        const Shell& ri = b.shells[b.onee_group_rep[gi]];
+                        const Shell& rj = b.shells[b.onee_group_rep[gj]];
+                        for (int a = 0; a < ri.nprim; ++a)
+                            for (int c = 0; c < rj.nprim; ++c) {
+                                const double ea = b.exps[ri.prim_offset + a], ec = b.exps[rj.prim_offset + c];
+                                const double pp = ea + ec, chi = ea * ec / pp;
+                                bound += std::fabs(c_first(ri, a) * c_first(rj, c)) * std::pow(kPi / pp, 1.5) *
+                                         std::exp(-chi * r2);
+                            }
+                    }
                 }
+                if (!keep) continue;
+                dev::OneePair op{};
+                op.A = i;
+                op.B = j;
+                if (b.shells[j].L > b.shells[i].L) std::swap(op.A, op.B);
+                op.do_st = 1;
+                op.do_v = (decay_eps <= 0.0 || bound >= decay_eps) ? 1 : 0;
+                out.push_back(op);
             }
-            if (!keep) continue;
-            dev::OneePair op{};
-            op.A = i;
-            op.B = j;
-            if (b.shells[j].L > b.shells[i].L) std::swap(op.A, op.B);
-            op.do_st = 1;
-            op.do_v = (decay_eps <= 0.0 || bound >= decay_eps) ? 1 : 0;
-            p.pairs.push_back(op);
         }
+    };
+    {
+        // the long rows first
+        std::atomic<std::size_t> next{0};
+        run_threads(ns < 64 ? 1 : std::min(host_threads(), part.size()), [&](std::size_t) {
+            for (std::size_t k; (k = next.fetch_add(1)) < part.size();) {
+                const std::size_t r = part.size() - 1 - k;
+                rows(static_cast<int>(r) * kRows, part[r]);
+            }
+        });
     }
+    for (const auto& v : part) p.pairs.insert(p.pairs.end(), v.begin(), v.end());
     p.nuc.clear();
     double zsum = 0.0;
     for (std::size_t a = 0; a < b.Z.size(); ++a) {
