@@ -28,9 +28,10 @@ namespace {
 
 template <typename R, int LC, int LD>
 void launch(const dev::PlanView& pv, const dev::ClassLaunch& cl, int sms, cudaStream_t s) {
-    // item slots per batch: 64, halved while the block needs more than 100 KB
+    // item slots per batch: 32 (64 take the shared memory of resident blocks),
+    // halved while the block needs more than 100 KB
     dev::RowsLayout lay;
-    int nb_items = 64;
+    int nb_items = 32;
     for (;;) {
         lay.init(cl.la, cl.lb, LC, LD, nb_items);
         if (lay.words * 8 <= 100 * 1024 || nb_items <= 16) break;

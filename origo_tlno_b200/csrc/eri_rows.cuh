@@ -26,13 +26,20 @@ namespace dev {
 
 constexpr int kRowCols = 16;      // ket columns per thread
 constexpr int kRowMaxGroups = 4;  // item groups per block
-constexpr int kRowTile = 4;       // outputs per thread and pass of the transfer products
 
 template <int LC, int LD>
 struct RowsKet {
     static constexpr int LCD = LC + LD, KS = LCD + 1, KSP = (KS + 1) / 2 * 2;
     static constexpr int OFC = ce_off(LC), NCS = ce_cum(LCD) - OFC;
     static constexpr int CH = (NCS + kRowCols - 1) / kRowCols, CC = (NCS + CH - 1) / CH;
+};
+
+// The sizes the digestion needs, those of the ket at compile time (its index
+// divisions then cost no division).
+template <int LC, int LD>
+struct RowsDims {
+    static constexpr int nc = ce_nsph(LC), nd = ce_nsph(LD), nscd = nc * nd;
+    int na, nb, nsab, off_P;
 };
 
 // Block shape and shared-memory layout (in elements of double) of a class.
@@ -67,7 +74,9 @@ struct RowsLayout {
         off_P = off_V + nsab * nscd;
         const int tail = off_P + na * nb + nc * nd + nb * nd + nb * nc + na * nd + na * nc;
         off_T = ((g_words > tail ? g_words : tail) + 1) & ~1;
-        words = (off_T + nas * ncs + 1) & ~1;
+        // odd row stride: the rows' threads store to different banks (the even
+        // stride of 16 was a 32-way conflict, two thirds of all wavefronts)
+        words = (off_T + nas * (ncs | 1) + 1) & ~1;
     }
 };
 
@@ -140,25 +149,35 @@ __device__ __forceinline__ void rows_dispatch(int chunk, const R* g, int slot, i
     }
 }
 
-// out[row * ld + s] = sum_k A(row, k) B(k, s), s < ns, kRowTile rows per
-// thread; A in shared memory or L1, B read once per kRowTile rows.
-template <typename FA, typename FB>
-__device__ __forceinline__ void rows_product(int nrows, int ns, int nk, FA&& a, FB&& b, double* out) {
-    const int blocks = (nrows + kRowTile - 1) / kRowTile;
+// out[row * ns + s] = sum_k A(row, k) B(k, s): TILE rows and one s per thread
+// and pass, so that a B value serves TILE sums; four steps of k in flight.
+template <int TILE, typename FA, typename FB>
+__device__ __forceinline__ void rows_product_tile(int nrows, int ns, int nk, FA&& a, FB&& b, double* out) {
+    const int blocks = (nrows + TILE - 1) / TILE;
     for (int e = threadIdx.x; e < blocks * ns; e += blockDim.x) {
-        const int rb = e / ns, s = e - rb * ns, r0 = rb * kRowTile;
-        double sum[kRowTile];
+        const int rb = e / ns, s = e - rb * ns, r0 = rb * TILE;
+        double sum[TILE];
 #pragma unroll
-        for (int t = 0; t < kRowTile; ++t) sum[t] = 0.0;
+        for (int t = 0; t < TILE; ++t) sum[t] = 0.0;
+#pragma unroll 4
         for (int k = 0; k < nk; ++k) {
             const double v = b(k, s);
 #pragma unroll
-            for (int t = 0; t < kRowTile; ++t) sum[t] += a(min(r0 + t, nrows - 1), k) * v;
+            for (int t = 0; t < TILE; ++t) sum[t] += a(min(r0 + t, nrows - 1), k) * v;
         }
 #pragma unroll
-        for (int t = 0; t < kRowTile; ++t)
+        for (int t = 0; t < TILE; ++t)
             if (r0 + t < nrows) out[(r0 + t) * ns + s] = sum[t];
     }
+}
+
+// The smallest tile that covers the product in one pass of the block.
+template <typename FA, typename FB>
+__device__ __forceinline__ void rows_product(int nrows, int ns, int nk, FA&& a, FB&& b, double* out) {
+    const int nt = blockDim.x;
+    if ((nrows + 1) / 2 * ns <= nt) rows_product_tile<2>(nrows, ns, nk, a, b, out);
+    else if ((nrows + 3) / 4 * ns <= nt) rows_product_tile<4>(nrows, ns, nk, a, b, out);
+    else rows_product_tile<6>(nrows, ns, nk, a, b, out);
 }
 
 template <typename R, int LC, int LD>
@@ -235,7 +254,7 @@ __device__ void rows_quartet(const PlanView& pv, const ClassLaunch& cl, const Ro
             for (int k = 0; k < K::CC; ++k) {
                 const int ic = chunk * K::CC + k;
                 if (ic < K::NCS) {
-                    R* t = T + row * K::NCS + ic;
+                    R* t = T + row * (K::NCS | 1) + ic;
                     *t = gi == 0 ? acc[k] : *t + acc[k];
                 }
             }
@@ -249,20 +268,29 @@ __device__ void rows_quartet(const PlanView& pv, const ClassLaunch& cl, const Ro
     const double* PKt = pv.proj + pv.proj_off[ket];
     double* X = sm + lay.off_X;
     double* V = sm + lay.off_V;
-    const int nscd = lay.nscd, nsab = lay.nsab;
-    rows_product(lay.nas, nscd, K::NCS, [&](int ia, int ic) { return double(T[ia * K::NCS + ic]); },
+    constexpr int nscd = RowsDims<LC, LD>::nscd;
+    const int nsab = lay.nsab;
+    rows_product(lay.nas, nscd, K::NCS, [&](int ia, int ic) { return double(T[ia * (K::NCS | 1) + ic]); },
                  [&](int ic, int s) { return __ldg(PKt + ic * nscd + s); }, X);
     __syncthreads();
     rows_product(nsab, nscd, lay.nas, [&](int sab, int ia) { return __ldg(PBt + ia * nsab + sab); },
                  [&](int ia, int s) { return X[ia * nscd + s]; }, V);
     __syncthreads();
-    block_digest(pv, cl, lay, sm, V, br, kr, bra, ket, jon, kon);
+    const RowsDims<LC, LD> dims{lay.na, lay.nb, nsab, lay.off_P};
+    block_digest(pv, cl, dims, sm, V, br, kr, bra, ket, jon, kon);
 }
+
+// Largest block of a ket class (bra (ff): 74 rows in whole warps per chunk) and
+// the resident blocks its registers are capped for: the kernel waits at
+// barriers and on L2, so 5 blocks of 128 threads beat 3 uncapped or 6 (f-shell
+// 14 atoms, its 20 classes: 15.0, 13.3 and 14.1 ms).
+__host__ __device__ constexpr int rows_max_threads(int ch) { return ch == 1 ? 128 : 96 * ch; }
+__host__ __device__ constexpr int rows_min_blocks(int ch) { return ch == 1 ? 5 : ch == 2 ? 3 : ch == 3 ? 2 : 1; }
 
 // Tiled schedule: tile = 1 bra pair x bk ket pairs, handed out by a block-wide
 // dynamic counter in parts of `part` kets (eri_generic_cta_jk_kernel).
 template <typename R, int LC, int LD>
-__global__ void __launch_bounds__(RowsKet<LC, LD>::CH > 3 ? 512 : 384)
+__global__ void __launch_bounds__(rows_max_threads(RowsKet<LC, LD>::CH), rows_min_blocks(RowsKet<LC, LD>::CH))
     eri_rows_jk_kernel(PlanView pv, ClassLaunch cl, int nb_items, int part) {
     extern __shared__ double smem[];
     RowsLayout lay;

@@ -108,6 +108,18 @@ double flops_per_prim(int a, int b, int c, int d) {
     const double ncart4 = double(n_cart(a)) * n_cart(b) * n_cart(c) * n_cart(d);
     return 30.0 + N * (40.0 + 15.0 + 3.0 * vaxis + 3.0 * ncart4);
 }
+// Classes with a compile-time kernel of 4 register slices that the
+// block-per-quartet kernel beats where the contraction is deep, that is where
+// the primitive loop outweighs its barriers: (dd|dp) 2.0 | 4.8 ms at 8.4
+// primitive quartets per quartet (f-shell 14 atoms), 8.5 | 5.2 ms at 1.2 (91
+// waters); (fp|dp) 2.5 | 4.7 ms at 11.7.  The projectors this needs (2-6 KB per
+// pair) are affordable up to a million pairs.
+constexpr double kBlockKernelPrims = 4.0;
+constexpr long long kBlockKernelPairs = 1000000;
+bool block_kernel_class(int la, int lb, int lc, int ld) {
+    return lc == 2 && ld == 1 && ((la == 2 && lb == 2) || (la == 3 && lb == 1));
+}
+
 // ---- tile shapes of the compile-time kernels ----
 // Work of a tile beside its primitive loop (geometry, transfers, digestion), in
 // primitive-quartet steps.
@@ -561,6 +573,16 @@ void build_plan(Plan2e& plan, const std::vector<const Basis*>& bases, std::vecto
     plan.combos.clear();
     plan.total_quartets = plan.total_prim_quartets = 0;
     plan.total_flops = 0.0;
+    // Mean primitive count of a pair class.
+    auto mean_nprim = [&](int X) {
+        double n = 0.0, sum = 0.0;
+        for (int m = 0; m < plan.n_mol; ++m)
+            for (int k = 0; k < plan.mol_pairs[m].cls_count[X]; ++k) {
+                sum += plan.pair_nprim[gbeg[m][X] + k];
+                n += 1.0;
+            }
+        return n > 0.0 ? sum / n : 0.0;
+    };
     // The class schedules are independent: built on host threads, uploaded in
     // class order.
     std::vector<ComboSchedule> todo;
@@ -582,7 +604,9 @@ void build_plan(Plan2e& plan, const std::vector<const Basis*>& bases, std::vecto
             cs.lc = lc; cs.ld = Y - lc * (lc + 1) / 2;
             const int combo_id = X * kMaxPairClasses + Y;
             cs.fast = has_fast_kernel(cs.la, cs.lb, cs.lc, cs.ld) &&
-                      !(combo_id < 256 && tune.force_generic[combo_id]);
+                      !(combo_id < 256 && tune.force_generic[combo_id]) &&
+                      !(block_kernel_class(cs.la, cs.lb, cs.lc, cs.ld) &&
+                        mean_nprim(X) * mean_nprim(Y) >= kBlockKernelPrims && plan.kept_pairs <= kBlockKernelPairs);
             cs.bb = cs.fast ? fast_kernel_bras(cs.la, cs.lb, cs.lc, cs.ld) : 1;
             cs.bk = cs.fast ? 32 : tune.generic_bk;
             todo.push_back(std::move(cs));
