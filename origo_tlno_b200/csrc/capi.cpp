@@ -167,9 +167,7 @@ void enqueue_jk(Plan2e& plan, const Tuning& tune, const BuildSpec& spec, const d
                 double* dK, long long total, int M_single, double* d_dmax, float* dD32, cudaStream_t s,
                 StreamFan* fan) {
     const bool want_j = spec.want_j, want_k = spec.want_k, mixed = spec.mixed;
-    TLNO_CUDA(cudaMemsetAsync(dJ, 0, sizeof(double) * total, s));
-    TLNO_CUDA(cudaMemsetAsync(dK, 0, sizeof(double) * total, s));
-    TLNO_CUDA(cudaMemsetAsync(plan.d_counters.ptr, 0, sizeof(int) * 2 * plan.combos.size(), s));
+    launch_clear_build(dJ, dK, total, plan.d_counters.as<int>(), static_cast<int>(2 * plan.combos.size()), s);
     if (mixed) launch_absmax_f32(dD, total, d_dmax, dD32, s);
     dev::DensityScreen den{};
     if (spec.den_mode) {
@@ -280,8 +278,7 @@ void enqueue_jk(Plan2e& plan, const Tuning& tune, const BuildSpec& spec, const d
         if (want_j) launch_symmetrize(dJ, plan.d_mol_mat_off.as<long long>(), plan.d_mol_M.as<int>(), plan.n_mol, maxm, s);
         if (want_k) launch_symmetrize(dK, plan.d_mol_mat_off.as<long long>(), plan.d_mol_M.as<int>(), plan.n_mol, maxm, s);
     } else {
-        if (want_j) launch_symmetrize_single(dJ, M_single, s);
-        if (want_k) launch_symmetrize_single(dK, M_single, s);
+        if (want_j || want_k) launch_symmetrize_single(want_j ? dJ : dK, want_j && want_k ? dK : nullptr, M_single, s);
     }
 }
 

@@ -130,7 +130,9 @@ T* upload(const std::vector<T>& v) {
 }
 
 // ---- utility kernels ----
-__global__ void symmetrize_kernel(double* X, int M) {
+// (X, and with two rows of blocks Y)
+__global__ void symmetrize_kernel(double* X0, double* Y, int M) {
+    double* X = blockIdx.y ? Y : X0;
     const long long n = (long long)M * M;
     for (long long e = blockIdx.x * (long long)blockDim.x + threadIdx.x; e < n; e += (long long)gridDim.x * blockDim.x) {
         const int i = static_cast<int>(e / M), j = static_cast<int>(e % M);
@@ -154,6 +156,16 @@ __global__ void symmetrize_batch_kernel(double* X, const long long* offs, const 
             Y[(long long)j * M + i] = v;
         }
     }
+}
+
+// Zeroes J, K and the schedule counters of a build in one launch.
+__global__ void clear_build_kernel(double* J, double* K, long long n, int* counters, int n_counters) {
+    const long long t = blockIdx.x * (long long)blockDim.x + threadIdx.x, nt = (long long)gridDim.x * blockDim.x;
+    for (long long e = t; e < n; e += nt) {
+        J[e] = 0.0;
+        K[e] = 0.0;
+    }
+    for (long long e = t; e < n_counters; e += nt) counters[e] = 0;
 }
 
 __global__ void boys_test_kernel(const double* x, int n, int maxn, double* out) {
@@ -652,10 +664,17 @@ void launch_symmetrize(double* X, const long long* offsets, const int* dims, int
     TLNO_CUDA(cudaGetLastError());
 }
 
-void launch_symmetrize_single(double* X, int M, cudaStream_t s) {
+void launch_symmetrize_single(double* X, double* Y, int M, cudaStream_t s) {
     const long long n = (long long)M * M;
-    const int grid = static_cast<int>(std::min<long long>((n + 255) / 256, sm_count() * 32));
-    symmetrize_kernel<<<grid, 256, 0, s>>>(X, M);
+    const dim3 grid(static_cast<int>(std::min<long long>((n + 255) / 256, sm_count() * 32)), Y ? 2 : 1);
+    symmetrize_kernel<<<grid, 256, 0, s>>>(X, Y, M);
+    TLNO_CUDA(cudaGetLastError());
+}
+
+void launch_clear_build(double* J, double* K, long long n, int* counters, int n_counters, cudaStream_t s) {
+    const long long m = std::max<long long>(n, n_counters);
+    const int grid = static_cast<int>(std::max<long long>(1, std::min<long long>((m + 255) / 256, sm_count() * 16)));
+    clear_build_kernel<<<grid, 256, 0, s>>>(J, K, n, counters, n_counters);
     TLNO_CUDA(cudaGetLastError());
 }
 

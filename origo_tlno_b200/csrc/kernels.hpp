@@ -62,7 +62,10 @@ void launch_onee(const dev::OneeLaunch& L, cudaStream_t s);
 // out = (X + X^T) / 2 for `count` stacked M x M blocks (offsets per block).
 void launch_symmetrize(double* X, const long long* offsets, const int* dims, int count, int max_m,
                        cudaStream_t s);
-void launch_symmetrize_single(double* X, int M, cudaStream_t s);
+// Symmetrises X and, when given, Y (both M x M) in one launch.
+void launch_symmetrize_single(double* X, double* Y, int M, cudaStream_t s);
+// Zeroes J, K (n elements each) and the schedule counters in one launch.
+void launch_clear_build(double* J, double* K, long long n, int* counters, int n_counters, cudaStream_t s);
 // *out = max |x_i| over n elements.
 void launch_absmax(const double* x, long long n, double* out, cudaStream_t s);
 // max|x| into *out and the FP32 copy x32 of x, one pass.
