@@ -14,16 +14,22 @@
 // compile time, so the accumulators stay in registers; TPQ is the smallest
 // power of two whose slice holds at most fast_acc_limit() accumulators.
 // The lanes of a split quartet take the ket and bra primitives in strides and
-// add their accumulators by shuffles; the first of them goes on.  A deep contraction is one long dependent chain per
-// lane (about 0.2 us per primitive quartet in FP64): with one lane per quartet
-// and few tiles the whole launch waited for single warps (24-atom organic
-// molecule, (ss|ss): 8.2 ms for 0.5 ms worth of work).
+// add their accumulators by shuffles; the first of them goes on.  A deep
+// contraction is one long dependent chain per lane (about 0.2 us per primitive
+// quartet in FP64): with one lane per quartet and few tiles the whole launch
+// waited for single warps (24-atom organic molecule, (ss|ss): 8.2 ms, 0.3 now).
 // Phase 2: ket HRR and ket spherical projection of the owned rows, written
 // to shared memory as (a0|cd)_sph rows.
 // Phase 3: after a barrier, each warp takes a share of the ket columns
 // (c,d)_sph, applies the bra HRR and projection and digests the finished
 // (ab|cd) column into J and K (J[ab] warp-reduced, the rest FP64 atomics
-// from per-thread partial sums).
+// from per-thread partial sums), from density values that were copied to
+// shared memory during phase 1.
+//
+// What bounds it (40 waters, (ps|ss) FP64 without digestion, ncu): about 150
+// issued instructions per primitive quartet of a warp, 64 of them FP64, at 16
+// resident warps; issue 46%, FP64 pipe 32%, the rest waits on FP64 latency
+// (2.9 cycles per issue) and L1/L2 loads (2.7).
 //
 // Arithmetic follows the reference's producer: contracted radial
 // accumulation, contracted-space HRR, final pair projection
@@ -526,16 +532,30 @@ __host__ __device__ constexpr bool fast_async() {
     return kSmem / (base + own) >= before;
 }
 
+// Whether J[ab] is summed over the lanes through shared memory, for 3 to 16
+// values (bra (ps), (pp), (ds), (dp)): NSAB stores and P loads instead of 5
+// shuffles per value (3 instructions each in FP64) and one atomic instruction
+// instead of NSAB.  91 waters, ms before -> after: FP64 (ps|ss) 44.4 -> 42.4,
+// (pp|ps) 31.6 -> 28.1, (dp|ss) 7.5 -> 5.9, (dp|ps) 16.8 -> 13.5; FP32 (dp|ps)
+// 11.0 -> 9.2.  Not the FP64 sliced classes, where the buffers cost a resident
+// CTA ((dp|pp) 20.9 -> 23.2).
+template <typename R, int LA, int LB, int LC, int LD>
+__host__ __device__ constexpr bool fast_jab_smem() {
+    using S = FastShape<LA, LB, LC, LD>;
+    return LA <= 2 && S::NSAB >= 3 && S::NSAB <= 16 && (S::TPQ == 1 || std::is_same<R, float>::value);
+}
+
 // Shared memory of one warp group's region (see the kernel), a multiple of 16
 // bytes.
 template <typename R, int LA, int LB, int LC, int LD>
 __host__ __device__ constexpr int fast_region_bytes() {
     using S = FastShape<LA, LB, LC, LD>;
-    if (!fast_async<R, LA, LB, LC, LD>()) return 0;
+    const int jab = fast_jab_smem<R, LA, LB, LC, LD>() ? S::TPQ * S::NSAB * 33 : 0;
+    if (!fast_async<R, LA, LB, LC, LD>()) return (jab * static_cast<int>(sizeof(R)) + 15) / 16 * 16;
     const int pre = fast_pre_mode<R, LA, LB, LC, LD>() == 2 ? S::PRE_VALS : 0;
     const int car = fast_carry_smem<R, LA, LB, LC, LD>() ? S::PRE_VALS : 0;
     const int bytes = (S::GB > 1 ? S::GB * (static_cast<int>(sizeof(PairRec)) + 4) : 0) +
-                      (S::GB * S::NSAB + 32 * (S::OWN_VALS + pre + car)) * static_cast<int>(sizeof(R));
+                      (S::GB * S::NSAB + 32 * (S::OWN_VALS + pre + car) + jab) * static_cast<int>(sizeof(R));
     return (bytes + 15) / 16 * 16;
 }
 
@@ -583,6 +603,8 @@ __global__ void __launch_bounds__(32 * FastShape<LA, LB, LC, LD>::WARPS, fast_mi
     R* dg = wdab + S::GB * S::NSAB;
     R* pre = dg + S::OWN_VALS * 32;
     R* carry = pre + (PRE_MODE == 2 ? S::PRE_VALS * 32 : 0);
+    R* jred = ASYNC ? carry + (fast_carry_smem<R, LA, LB, LC, LD>() ? S::PRE_VALS * 32 : 0)
+                    : reinterpret_cast<R*>(wsm);
     int staged = -1;               // block whose bras are staged
     double qmax = 0.0, qmin = 0.0; // bounds of the staged bras
     int imax = 0;                  // largest class index of the staged bras
@@ -783,6 +805,9 @@ __global__ void __launch_bounds__(32 * FastShape<LA, LB, LC, LD>::WARPS, fast_mi
             constexpr int BX = GROUP ? 0 : S::NSA * (S::NSC + S::NSD);  // first D[b,c] slot of a lane
             constexpr int CX = BX + S::NSB * (S::NSC + S::NSD);         // first D[c,d] slot
             if constexpr (ASYNC) {
+                // the slots of the tile before have been read by every lane
+                // (a sliced quartet ends with a group barrier)
+                if constexpr (!GROUP && S::TPQ == 1) __syncwarp();
                 auto copy = [&](int k, int r, int c, int off) {
                     if (S::TPQ == 1 || k % S::TPQ == g) async_copy(dg + k * 32 + lane, dp(r, c, off));
                 };
@@ -993,12 +1018,33 @@ __global__ void __launch_bounds__(32 * FastShape<LA, LB, LC, LD>::WARPS, fast_mi
             }
             if (cl.want_j) {
                 // J[ab]: every lane of the warp shares the bra pair.
+                if constexpr (fast_jab_smem<R, LA, LB, LC, LD>()) {
+                    // summed over the lanes through shared memory: P lanes per
+                    // part of the row, P = 4, 8 or 16 >= NSAB
+                    constexpr int P = S::NSAB <= 4 ? 4 : S::NSAB <= 8 ? 8 : 16;
+                    R* red = jred + g * (S::NSAB * 33);
 #pragma unroll
-                for (int e = 0; e < S::NSAB; ++e) {
-                    R s = fj * jab[e];
+                    for (int e = 0; e < S::NSAB; ++e) red[e * 33 + lane] = fj * jab[e];
+                    __syncwarp();
+                    const int e = lane % P;
+                    R s = R(0);
+                    if (e < S::NSAB) {
+                        const R* row = red + e * 33 + lane / P * P;
 #pragma unroll
-                    for (int o = 16; o > 0; o >>= 1) s += __shfl_xor_sync(0xffffffffu, s, o);
-                    if (lane == 0 && s != R(0)) add_j(a0 + e / S::NSB, b0, e % S::NSB, s);
+                        for (int k = 0; k < P; ++k) s += row[k];
+                    }
+#pragma unroll
+                    for (int o = 16; o >= P; o >>= 1) s += __shfl_xor_sync(0xffffffffu, s, o);
+                    if (lane < S::NSAB && s != R(0)) add_j(a0 + lane / S::NSB, b0 + lane % S::NSB, 0, s);
+                    __syncwarp();
+                } else {
+#pragma unroll
+                    for (int e = 0; e < S::NSAB; ++e) {
+                        R s = fj * jab[e];
+#pragma unroll
+                        for (int o = 16; o > 0; o >>= 1) s += __shfl_xor_sync(0xffffffffu, s, o);
+                        if (lane == 0 && s != R(0)) add_j(a0 + e / S::NSB, b0, e % S::NSB, s);
+                    }
                 }
             }
             if constexpr (S::TPQ > 1) group_sync(bar_id, bar_n);

@@ -14,7 +14,7 @@ namespace tlno_gpu {
 // Largest pair-projector table a plan keeps on the device; above it the
 // generic classes run the warp-per-quartet kernel, which builds projectors
 // per quartet.
-constexpr long long kMaxProjectorBytes = 8LL << 30;
+constexpr long long kMaxProjectorBytes = 16LL << 30;
 
 struct Tuning {
     int generic_bk = 64;    // ket pairs per tile of the warp-per-quartet kernel
