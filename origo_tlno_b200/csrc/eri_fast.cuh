@@ -26,10 +26,11 @@
 // from per-thread partial sums), from density values that were copied to
 // shared memory during phase 1.
 //
-// What bounds it (40 waters, (ps|ss) FP64 without digestion, ncu): about 150
-// issued instructions per primitive quartet of a warp, 64 of them FP64, at 16
-// resident warps; issue 46%, FP64 pipe 32%, the rest waits on FP64 latency
-// (2.9 cycles per issue) and L1/L2 loads (2.7).
+// What bounds it (40 waters, (ps|ss) FP64, ncu): about 130 issued instructions
+// per primitive quartet of a warp, 55 of them FP64, at 16 resident warps; issue
+// 43%, FP64 pipe 36%, the rest waits on FP64 latency (2.7 cycles per issue) and
+// L1/L2 loads (3.8); with digestion the L1 data pipe is at 76% of its wavefront
+// rate (scattered atomics and density copies).
 //
 // Arithmetic follows the reference's producer: contracted radial
 // accumulation, contracted-space HRR, final pair projection
