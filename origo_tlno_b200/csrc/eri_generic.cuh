@@ -409,13 +409,14 @@ __global__ void eri_generic_jk_kernel(PlanView pv, ClassLaunch cl) {
 }
 
 // ---------------------------------------------------------------------------
-// CTA-cooperative J/K kernel for the classes the compile-time kernels do not
-// cover (two f shells, or deep d/f slices).  One thread block works on one
-// contracted quartet at a time, so a class whose radial block, transfer
-// products and 2-D tables need tens of KB of shared memory keeps 4-8 warps
-// busy per block instead of one warp per block.  The HRR + spherical
-// projectors of both pairs come precomputed from the plan (one per shell
-// pair, built once per plan by pair_projector_kernel).
+// CTA-cooperative J/K kernel of the classes that neither a compile-time kernel
+// nor the row kernel (eri_rows.cuh) covers: a g shell, or an (ss|, (ps| bra
+// forced off its compile-time kernel.  One thread block works on one contracted
+// quartet at a time, so a class whose radial block, transfer products and 2-D
+// tables need tens of KB of shared memory keeps 4-8 warps busy per block instead
+// of one warp per block.  The HRR + spherical projectors of both pairs come
+// precomputed from the plan (one per shell pair, built once per plan by
+// pair_projector_kernel).
 //
 // Shared memory (doubles): region0 = max(NB item slots x 3 2-D tables,
 // X + V + the six density blocks), then the radial block T.
@@ -573,9 +574,9 @@ __device__ void generic_quartet_cta(const PlanView& pv, const ClassLaunch& cl, c
 
 // Tiled schedule (J/K mode), one quartet per block at a time: tile = 1 bra
 // pair x bk ket pairs, handed out by a block-wide dynamic counter in parts of
-// `part` kets.  A quartet of two f shells takes a block 10-50 us, so whole
-// tiles of 64 left most SMs idle on small molecules (f-shell 14 atoms,
-// (ff|ff): 31 tiles, 393 quartets, 1.66 ms).
+// `part` kets: with whole tiles of 64 most SMs idled on small molecules (when
+// this kernel ran them, (ff|ff) of 14 f-shell atoms, 31 tiles of 393 quartets:
+// 1.66 -> 0.27 ms).
 template <typename R>
 __global__ void eri_generic_cta_jk_kernel(PlanView pv, ClassLaunch cl, int nb_items, int part) {
     extern __shared__ double smem[];
