@@ -11,6 +11,7 @@
 #include <cmath>
 #include <cstring>
 #include <functional>
+#include <map>
 #include <memory>
 #include <string>
 #include <vector>
@@ -136,6 +137,11 @@ void StreamFan::ensure(int n_aux) {
         TLNO_CUDA(cudaEventCreateWithFlags(&e, cudaEventDisableTiming));
         ev.push_back(e);
     }
+}
+
+StreamFan& thread_fan(int device) {
+    thread_local std::map<int, StreamFan> fans;
+    return fans[device];
 }
 
 StreamFan::~StreamFan() {
@@ -421,7 +427,7 @@ void run_jk(tlno_gpu_context* ctx, const double* density, double* J, double* K, 
         const bool pj = den ? out_j : (out_j || want_g);
         const bool pk = den ? out_k : (out_k || want_g);
         enqueue_jk(*ctx->plan, ctx->tune, spec_from(eo, pj, pk, mixed, false), dD, dJ, dK, n, M,
-                   ctx->w.dmax.as<double>(), d32, s, &ctx->fan);
+                   ctx->w.dmax.as<double>(), d32, s, &thread_fan(ctx->device));
         if (!dev_ptrs) {
             if (out_j) TLNO_CUDA(cudaMemcpyAsync(J, dJ, sizeof(double) * n, cudaMemcpyDeviceToHost, s));
             if (out_k) TLNO_CUDA(cudaMemcpyAsync(K, dK, sizeof(double) * n, cudaMemcpyDeviceToHost, s));
@@ -434,7 +440,7 @@ void run_jk(tlno_gpu_context* ctx, const double* density, double* J, double* K, 
             gJ = ctx->w.J.as<double>();
             gK = ctx->w.K.as<double>();
             enqueue_jk(*ctx->plan, ctx->tune, spec_from(eo, true, true, mixed, true), dD, gJ, gK, n, M,
-                       ctx->w.dmax.as<double>(), d32, s, &ctx->fan);
+                       ctx->w.dmax.as<double>(), d32, s, &thread_fan(ctx->device));
         }
         double* dG = G;
         if (!dev_ptrs) {
@@ -865,7 +871,7 @@ int tlno_gpu_jk_graph_capture(tlno_gpu_context* ctx, const double* d_density, do
         TLNO_CUDA(cudaStreamBeginCapture(ctx->stream, cudaStreamCaptureModeThreadLocal));
         try {
             enqueue_jk(*ctx->plan, ctx->tune, spec, d_density, d_J, d_K, n, M, ctx->w.dmax.as<double>(), d32,
-                       ctx->stream, &ctx->fan);
+                       ctx->stream, &thread_fan(ctx->device));
         } catch (...) {
             cudaGraph_t g = nullptr;
             cudaStreamEndCapture(ctx->stream, &g);
@@ -1173,7 +1179,7 @@ int tlno_gpu_batch_jk(tlno_gpu_batch* b, const double* density, double* J, doubl
         validate_build_combination(b->screening);
         if (b->screening.density_threshold > 0.0) ensure_density_tables(b->plan);
         enqueue_jk(b->plan, b->tune, spec_from(b->screening, true, true, flags & TLNO_GPU_MIXED, false), dD, dJ, dK,
-                   b->total, 0, b->w.dmax.as<double>(), d32, s, &b->fan);
+                   b->total, 0, b->w.dmax.as<double>(), d32, s, &thread_fan(b->device));
         if (!dev_ptrs) {
             TLNO_CUDA(cudaMemcpyAsync(J, dJ, sizeof(double) * b->total, cudaMemcpyDeviceToHost, s));
             TLNO_CUDA(cudaMemcpyAsync(K, dK, sizeof(double) * b->total, cudaMemcpyDeviceToHost, s));
@@ -1200,7 +1206,7 @@ int tlno_gpu_batch_graph_capture(tlno_gpu_batch* b, const double* d_density, dou
         TLNO_CUDA(cudaStreamBeginCapture(b->stream, cudaStreamCaptureModeThreadLocal));
         try {
             enqueue_jk(b->plan, b->tune, spec, d_density, d_J, d_K, b->total, 0, b->w.dmax.as<double>(), d32,
-                       b->stream, &b->fan);
+                       b->stream, &thread_fan(b->device));
         } catch (...) {
             cudaGraph_t g = nullptr;
             cudaStreamEndCapture(b->stream, &g);

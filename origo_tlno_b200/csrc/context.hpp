@@ -29,6 +29,12 @@ struct StreamFan {
     ~StreamFan();
 };
 
+// The calling thread's fan on a device, made on first use and given back when
+// the thread ends.  A build uses it only while its call enqueues (direct calls
+// then wait for their work; a captured graph keeps no stream), so the contexts
+// and batches of one thread share it and threads never do.
+StreamFan& thread_fan(int device);
+
 struct JkWork {
     DeviceBuffer D, J, K, G, dmax, status;
     DeviceBuffer D32;  // FP32 copy of the density for the FP32 kernels (mixed builds)
@@ -48,7 +54,6 @@ struct tlno_gpu_context {
     tlno_gpu::DeviceBuffer d_shell_xyz, d_shell_L, d_shell_nprim, d_shell_prim, d_shell_sph, d_exps, d_crad;
     tlno_gpu::DeviceBuffer d_comp_coef, d_comp_off;
     tlno_gpu::JkWork w;
-    tlno_gpu::StreamFan fan;
     tlno_gpu::DeviceBuffer d_S, d_T, d_V;
     cudaGraph_t graph = nullptr;
     cudaGraphExec_t graph_exec = nullptr;
@@ -69,7 +74,6 @@ struct tlno_gpu_batch {
     tlno_gpu_screening screening{};
     tlno_gpu::Tuning tune;
     tlno_gpu::JkWork w;
-    tlno_gpu::StreamFan fan;
     long long total = 0;
     cudaGraph_t graph = nullptr;
     cudaGraphExec_t graph_exec = nullptr;
