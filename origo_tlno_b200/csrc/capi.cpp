@@ -340,8 +340,7 @@ void replan(tlno_gpu_context* ctx, const tlno_gpu_screening& o) {
 namespace tlno_gpu {
 
 std::unique_ptr<Plan2e> make_plan(const tlno_gpu_context* ctx, const tlno_gpu_screening& o) {
-    if (ctx->basis.n_sph > 65535)
-        throw Error(TLNO_GPU_E_INVALID, "eri_ao_tensor_hgp: direct J/K pair tables assume M <= 65535.");
+    check_function_count(ctx->basis);  // before the pair lists
     auto plan = std::make_unique<Plan2e>();
     std::vector<MolPairs> mp;
     const double tau = o.decay_threshold > 0.0 ? o.decay_threshold : o.integral_threshold;
@@ -1102,6 +1101,7 @@ int tlno_gpu_batch_create(int n_mol, tlno_gpu_context* const* ctxs, const tlno_g
         for (int m = 0; m < n_mol; ++m) {
             if (!ctxs[m] || ctxs[m]->device != b->device)
                 throw Error(TLNO_GPU_E_INVALID, "tlno_gpu: batch contexts must share one device");
+            check_function_count(ctxs[m]->basis);
             b->bases.push_back(ctxs[m]->basis);
         }
         for (int m = 0; m < n_mol; ++m)

@@ -431,8 +431,13 @@ dev::PlanView Plan2e::view() const {
     return pv;
 }
 
+void check_function_count(const Basis& b) {
+    if (b.n_sph > 65535) throw Error(-1, "eri_ao_tensor_hgp: direct J/K pair tables assume M <= 65535.");
+}
+
 void build_plan(Plan2e& plan, const std::vector<const Basis*>& bases, std::vector<MolPairs>&& pairs,
                 double tau, const Tuning& tune, cudaStream_t s) {
+    for (const Basis* b : bases) check_function_count(*b);
     plan.tau = tau;
     plan.n_mol = static_cast<int>(bases.size());
     plan.mol_pairs = std::move(pairs);

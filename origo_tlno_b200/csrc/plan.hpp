@@ -100,6 +100,9 @@ public:
 // decay indicator K_A K_B exp(-mu_min |AB|^2) (rys_engine.ipp:2205-2241) and
 // screens the pair products against decay instead of tau.
 MolPairs build_mol_pairs(const Basis& b, double tau, cudaStream_t s, double decay = 0.0);
+// Refuses a basis beyond the 65535 functions that the J/K kernels' 32-bit
+// matrix indices hold; every plan, of a context or a batch, goes through it.
+void check_function_count(const Basis& b);
 // Allocates the density-screen tables of a plan (idempotent).
 void ensure_density_tables(Plan2e& plan);
 
