@@ -148,6 +148,10 @@ int tlno_gpu_jk(tlno_gpu_context* ctx, const double* density, double* J, double*
  * density predicate.  mixed_threshold keeps the context's value. */
 int tlno_gpu_jk_with_options(tlno_gpu_context* ctx, const double* density, double* J, double* K,
                              double* G, int flags, const tlno_gpu_screening* options);
+/* Testing hook: the next J/K build of the context (direct call or graph
+ * capture) fails on the host after `launches` of its class launches; what was
+ * queued before completes in the order of the context's stream. */
+int tlno_gpu_fail_next_build(tlno_gpu_context* ctx, int launches);
 
 /* ERI checksum stream: the sum of every canonical unique spherical ERI
  * (ij|kl), i >= j, k >= l, ij >= kl over AO pair indices, whose shell

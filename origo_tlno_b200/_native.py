@@ -97,6 +97,7 @@ def lib() -> C.CDLL:
         "tlno_gpu_plan_profile": (C.c_int, [_vp, C.POINTER(Profile)]),
         "tlno_gpu_jk": (C.c_int, [_vp, _vp, _vp, _vp, _vp, C.c_int]),
         "tlno_gpu_jk_with_options": (C.c_int, [_vp, _vp, _vp, _vp, _vp, C.c_int, C.POINTER(Screening)]),
+        "tlno_gpu_fail_next_build": (C.c_int, [_vp, C.c_int]),
         "tlno_gpu_eri_checksum": (C.c_int, [_vp, _dp, _dp]),
         "tlno_gpu_incremental_create": (C.c_int, [_vp, C.POINTER(IncrementalOptions), C.POINTER(_vp)]),
         "tlno_gpu_incremental_destroy": (None, [_vp]),
@@ -162,7 +163,8 @@ def ptr(a) -> int:
 EXPORTED = [
     "tlno_gpu_last_error", "tlno_gpu_version", "tlno_gpu_device_count", "tlno_gpu_create",
     "tlno_gpu_create_from_components", "tlno_gpu_destroy", "tlno_gpu_n_sph", "tlno_gpu_n_shells",
-    "tlno_gpu_plan", "tlno_gpu_plan_profile", "tlno_gpu_jk", "tlno_gpu_jk_with_options", "tlno_gpu_eri_checksum",
+    "tlno_gpu_plan", "tlno_gpu_plan_profile", "tlno_gpu_jk", "tlno_gpu_jk_with_options", "tlno_gpu_fail_next_build",
+    "tlno_gpu_eri_checksum",
     "tlno_gpu_incremental_create", "tlno_gpu_incremental_destroy", "tlno_gpu_incremental_update",
     "tlno_gpu_incremental_g", "tlno_gpu_incremental_density", "tlno_gpu_incremental_info_get",
     "tlno_gpu_incremental_reset", "tlno_gpu_incremental_fail_next_update",

@@ -14,6 +14,7 @@
 #include <map>
 #include <memory>
 #include <string>
+#include <utility>
 #include <vector>
 
 #include "engine.hpp"
@@ -151,6 +152,34 @@ StreamFan::~StreamFan() {
     for (cudaEvent_t e : ev) cudaEventDestroy(e);
 }
 
+// Fork of a build's stream onto auxiliary streams.  The branches are joined on
+// every way out: after a failure halfway the launches already queued still add
+// into the caller's J and K, and waiting for the build's stream has to cover them.
+StreamBranches::StreamBranches(StreamFan* fan, cudaStream_t s, int n) : fan_(fan), st(1, s) {
+    if (n <= 1) return;
+    fan->ensure(n - 1);
+    TLNO_CUDA(cudaEventRecord(fan->ev[0], s));
+    for (int k = 0; k < n - 1; ++k) {
+        TLNO_CUDA(cudaStreamWaitEvent(fan->aux[k], fan->ev[0], 0));
+        st.push_back(fan->aux[k]);
+    }
+}
+
+void StreamBranches::join() {
+    while (st.size() > 1) {
+        const std::size_t k = st.size() - 1;
+        TLNO_CUDA(cudaEventRecord(fan_->ev[k], st[k]));
+        TLNO_CUDA(cudaStreamWaitEvent(st[0], fan_->ev[k], 0));
+        st.pop_back();
+    }
+}
+
+StreamBranches::~StreamBranches() {
+    for (std::size_t k = 1; k < st.size(); ++k)
+        if (cudaEventRecord(fan_->ev[k], st[k]) != cudaSuccess || cudaStreamWaitEvent(st[0], fan_->ev[k], 0) != cudaSuccess)
+            cudaGetLastError();
+}
+
 // Streams a build's launches spread over: as tuned, else up to 8 for a build
 // whose class launches are too short to fill the chip each (below
 // kFanMaxFlops), where their latencies overlap; a longer build runs them one
@@ -213,15 +242,9 @@ void enqueue_jk(Plan2e& plan, const Tuning& tune, const BuildSpec& spec, const d
     // so far (largest classes first), join before the symmetrisation.  J and K
     // take FP64 atomics, so the order is free.
     const int nst = fan ? fan_streams(plan, tune, launches.size()) : 1;
-    std::vector<cudaStream_t> st(1, s);
+    StreamBranches branches(fan, s, nst);
     std::vector<int> stream_of(launches.size(), 0);
     if (nst > 1) {
-        fan->ensure(nst - 1);
-        TLNO_CUDA(cudaEventRecord(fan->ev[0], s));
-        for (int k = 0; k < nst - 1; ++k) {
-            TLNO_CUDA(cudaStreamWaitEvent(fan->aux[k], fan->ev[0], 0));
-            st.push_back(fan->aux[k]);
-        }
         std::stable_sort(launches.begin(), launches.end(), [&](const Launch& x, const Launch& y) {
             return plan.combos[x.ci].flops > plan.combos[y.ci].flops;
         });
@@ -236,7 +259,9 @@ void enqueue_jk(Plan2e& plan, const Tuning& tune, const BuildSpec& spec, const d
         const std::size_t ci = launches[li].ci;
         const int pass = launches[li].pass;
         ComboSchedule& cs = plan.combos[ci];
-        cudaStream_t cs_stream = st[stream_of[li]];
+        cudaStream_t cs_stream = branches.st[stream_of[li]];
+        if (static_cast<int>(li) == spec.fail_after)
+            throw Error(TLNO_GPU_E_STATE, "tlno_gpu: injected failure between the class launches");
         dev::ClassLaunch cl{};
         cl.la = cs.la; cl.lb = cs.lb; cl.lc = cs.lc; cl.ld = cs.ld;
         cl.same = (cs.X == cs.Y);
@@ -272,12 +297,7 @@ void enqueue_jk(Plan2e& plan, const Tuning& tune, const BuildSpec& spec, const d
         else
             launch_eri_jk_generic(pv, cl, fp32, tune.generic_warps, grid, cs_stream);
     }
-    if (nst > 1) {
-        for (int k = 0; k < nst - 1; ++k) {
-            TLNO_CUDA(cudaEventRecord(fan->ev[k + 1], fan->aux[k]));
-            TLNO_CUDA(cudaStreamWaitEvent(s, fan->ev[k + 1], 0));
-        }
-    }
+    branches.join();
     if (plan.n_mol > 1) {
         int maxm = 0;
         for (int m : plan.mol_M) maxm = std::max(maxm, m);
@@ -425,7 +445,9 @@ void run_jk(tlno_gpu_context* ctx, const double* density, double* J, double* K, 
     if (pass_jk) {
         const bool pj = den ? out_j : (out_j || want_g);
         const bool pk = den ? out_k : (out_k || want_g);
-        enqueue_jk(*ctx->plan, ctx->tune, spec_from(eo, pj, pk, mixed, false), dD, dJ, dK, n, M,
+        BuildSpec spec = spec_from(eo, pj, pk, mixed, false);
+        spec.fail_after = std::exchange(ctx->fail_after, -1);
+        enqueue_jk(*ctx->plan, ctx->tune, spec, dD, dJ, dK, n, M,
                    ctx->w.dmax.as<double>(), d32, s, &thread_fan(ctx->device));
         if (!dev_ptrs) {
             if (out_j) TLNO_CUDA(cudaMemcpyAsync(J, dJ, sizeof(double) * n, cudaMemcpyDeviceToHost, s));
@@ -545,6 +567,13 @@ int tlno_gpu_jk_with_options(tlno_gpu_context* ctx, const double* density, doubl
         if (!ctx || !options) throw Error(TLNO_GPU_E_INVALID, "tlno_gpu: null argument");
         validate_screening(*options);
         run_jk(ctx, density, J, K, G, flags, *options);
+    });
+}
+
+int tlno_gpu_fail_next_build(tlno_gpu_context* ctx, int launches) {
+    return guarded([&] {
+        if (!ctx || launches < 0) throw Error(TLNO_GPU_E_INVALID, "tlno_gpu: invalid failure position");
+        ctx->fail_after = launches;
     });
 }
 
@@ -865,8 +894,9 @@ int tlno_gpu_jk_graph_capture(tlno_gpu_context* ctx, const double* d_density, do
         }
         validate_build_combination(ctx->screening);
         if (ctx->screening.density_threshold > 0.0) ensure_density_tables(*ctx->plan);
-        const BuildSpec spec = spec_from(ctx->screening, want_j, want_k, flags & TLNO_GPU_MIXED,
-                                         (flags & TLNO_GPU_WANT_G) != 0);
+        BuildSpec spec = spec_from(ctx->screening, want_j, want_k, flags & TLNO_GPU_MIXED,
+                                   (flags & TLNO_GPU_WANT_G) != 0);
+        spec.fail_after = std::exchange(ctx->fail_after, -1);
         TLNO_CUDA(cudaStreamBeginCapture(ctx->stream, cudaStreamCaptureModeThreadLocal));
         try {
             enqueue_jk(*ctx->plan, ctx->tune, spec, d_density, d_J, d_K, n, M, ctx->w.dmax.as<double>(), d32,

@@ -35,6 +35,23 @@ struct StreamFan {
 // and batches of one thread share it and threads never do.
 StreamFan& thread_fan(int device);
 
+// A build's stream forked onto n - 1 auxiliary streams of a fan: st[0] is the
+// build's own, joined again by join() or, after a failure, by the destructor.
+class StreamBranches {
+public:
+    StreamBranches(StreamFan* fan, cudaStream_t s, int n);
+    ~StreamBranches();
+    StreamBranches(const StreamBranches&) = delete;
+    StreamBranches& operator=(const StreamBranches&) = delete;
+    void join();
+
+private:
+    StreamFan* fan_;
+
+public:
+    std::vector<cudaStream_t> st;
+};
+
 struct JkWork {
     DeviceBuffer D, J, K, G, dmax, status;
     DeviceBuffer D32;  // FP32 copy of the density for the FP32 kernels (mixed builds)
@@ -50,6 +67,7 @@ struct tlno_gpu_context {
     tlno_gpu::Tuning tune;
     tlno_gpu::OneePlan onee;
     int onee_state = -1;  // screening flag the 1e plan was built with
+    int fail_after = -1;   // testing hook: the next build fails after this many class launches
     double onee_decay_eps = 1e-15, onee_nuclear_eps = 1e-15;
     tlno_gpu::DeviceBuffer d_shell_xyz, d_shell_L, d_shell_nprim, d_shell_prim, d_shell_sph, d_exps, d_crad;
     tlno_gpu::DeviceBuffer d_comp_coef, d_comp_off;

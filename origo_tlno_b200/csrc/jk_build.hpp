@@ -40,6 +40,7 @@ struct BuildSpec {
     int den_mode = 0;      // 0 off; 1 J and K predicates apart; 2 fused G predicate
     double den_thr = 0.0;  // density_threshold
     double fs_thr2 = 0.0;  // primitive FASTSCHWARZ threshold squared
+    int fail_after = -1;   // testing hook: fail after this many class launches
 };
 BuildSpec spec_from(const tlno_gpu_screening& o, bool want_j, bool want_k, bool mixed, bool fused_g);
 

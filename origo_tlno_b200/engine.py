@@ -162,6 +162,11 @@ class Context:
         flags = N.WANT_J | N.WANT_K | N.DEVICE_PTRS | (N.MIXED if mixed else 0) | (0 if validate else N.NO_VALIDATE)
         N.check(N.lib().tlno_gpu_jk(self.h, d_density_ptr, d_J, d_K, None, flags))
 
+    def fail_next_build(self, launches: int):
+        """Testing hook: the next J/K build or capture fails on the host after
+        `launches` class launches."""
+        N.check(N.lib().tlno_gpu_fail_next_build(self.h, launches))
+
     def eri_checksum(self):
         """(checksum, device ms) of the ERI stream: the sum of the canonical
         unique spherical ERIs that pass the plan's screen."""
