@@ -274,7 +274,8 @@ int tlno_gpu_boys(int device, int n, int maxn, const double* x, double* out);
  * (rys_engine.ipp:3823-3838).  fp32 selects the evaluation path of the
  * kernels: 0 = FP64 tables (the reference's 0.01-grid interpolant),
  * 1 = FP32 tables, 2 = the FP32 interval polynomials of the mixed-precision
- * kernels (nroots <= 3). */
+ * kernels (nroots <= 3); 3 and 4 = what the compile-time kernels run in FP64 and
+ * in their FP32 pass (nroots <= 5; a NaN argument is passed on to them). */
 int tlno_gpu_rys(int device, int n, int nroots, const double* T, double* roots, double* weights,
                  int fp32);
 

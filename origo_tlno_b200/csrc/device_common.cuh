@@ -176,10 +176,11 @@ __device__ __forceinline__ float rsqrt_pos(float x) {
     return y;
 }
 
-// Asymptotic Rys roots and weights (T >= tmax(N)).
+// Asymptotic Rys roots and weights (T >= tmax(N)).  A NaN stays one.
 template <typename R, int N>
 __device__ __forceinline__ void rys_asymptotic(R T, R* root, R* weight) {
-    const R x = fmin(T, sizeof(R) == 4 ? R(1e37) : R(1e300));
+    constexpr R cap = sizeof(R) == 4 ? R(1e37) : R(1e300);
+    const R x = T > cap ? cap : T;
     R s = rsqrt_pos(x);
     if (sizeof(R) == 4) s = fma(R(0.5) * s, fma(-x * s, s, R(1)), s);
     R inv = s * s;
@@ -191,10 +192,12 @@ __device__ __forceinline__ void rys_asymptotic(R T, R* root, R* weight) {
     }
 }
 
-// All N roots at once (compile-time N).
+// All N roots at once (compile-time N).  The table is read only for T < tmax:
+// a NaN (p q overflows FP32 from exponents of 2e19) takes the asymptotic form,
+// its bits would make a grid index outside the table.
 template <typename R, int N>
 __device__ __forceinline__ void rys_roots_all(R T, R* root, R* weight) {
-    if (T >= R(c_tabs.tmax[N])) {
+    if (!(T < R(c_tabs.tmax[N]))) {
         rys_asymptotic<R, N>(T, root, weight);
         return;
     }
@@ -240,7 +243,7 @@ __device__ __forceinline__ void rys_roots_all(R T, R* root, R* weight) {
 template <int N>
 __device__ __forceinline__ void rys_roots_smem32(float T, const float* __restrict__ table, float* root,
                                                  float* weight) {
-    if (T >= float(c_tabs.tmax[N])) {
+    if (!(T < float(c_tabs.tmax[N]))) {  // or a NaN, as in rys_roots_all
         rys_asymptotic<float, N>(T, root, weight);
         return;
     }

@@ -202,6 +202,30 @@ __global__ void rys_interval_test_kernel(const double* T, int n, int mode, doubl
     }
 }
 
+// Test hook of the compile-time kernels' root evaluation: FP64 (mode 3), or
+// their FP32 pass (mode 4: interval polynomials for N <= 3, FP64 roots of the
+// FP32 argument above).
+template <int N>
+__global__ void rys_fast_test_kernel(const double* T, int n, int mode, double* roots, double* weights) {
+    const int i = blockIdx.x * blockDim.x + threadIdx.x;
+    if (i >= n) return;
+    double r[N], w[N];
+    bool done = false;
+    if constexpr (N <= kRys32MaxN) {
+        if (mode == 4) {
+            float rf[N], wf[N];
+            rys_roots_smem32<N>(float(T[i]), c_tabs.rys32[N], rf, wf);
+            for (int k = 0; k < N; ++k) r[k] = rf[k], w[k] = wf[k];
+            done = true;
+        }
+    }
+    if (!done) rys_roots_all<double, N>(mode == 4 ? double(float(T[i])) : T[i], r, w);
+    for (int k = 0; k < N; ++k) {
+        roots[(long long)i * N + k] = r[k];
+        weights[(long long)i * N + k] = w[k];
+    }
+}
+
 __global__ void absmax_kernel(const double* x, long long n, double* out) {
     __shared__ double red[32];
     double m = 0.0;
@@ -767,6 +791,19 @@ void launch_boys_test(const double* x, int n, int maxn, double* out, cudaStream_
 
 void launch_rys_test(const double* t, int n, int nroots, int fp32, double* roots, double* weights,
                      cudaStream_t s) {
+    if (fp32 >= 3) {
+        const int g = (n + 127) / 128;
+        switch (nroots) {
+            case 1: rys_fast_test_kernel<1><<<g, 128, 0, s>>>(t, n, fp32, roots, weights); break;
+            case 2: rys_fast_test_kernel<2><<<g, 128, 0, s>>>(t, n, fp32, roots, weights); break;
+            case 3: rys_fast_test_kernel<3><<<g, 128, 0, s>>>(t, n, fp32, roots, weights); break;
+            case 4: rys_fast_test_kernel<4><<<g, 128, 0, s>>>(t, n, fp32, roots, weights); break;
+            case 5: rys_fast_test_kernel<5><<<g, 128, 0, s>>>(t, n, fp32, roots, weights); break;
+            default: break;
+        }
+        TLNO_CUDA(cudaGetLastError());
+        return;
+    }
     if (fp32 >= 2) {
         const int g = (n + 127) / 128;
         switch (nroots) {

@@ -510,12 +510,14 @@ def boys(x, maxn: int, device: int = 0) -> np.ndarray:
     return out
 
 
-RYS_PATHS = {"fp64_table": 0, "fp32_table": 1, "fp32_interval": 2}
+RYS_PATHS = {"fp64_table": 0, "fp32_table": 1, "fp32_interval": 2, "fp64_fast": 3, "fp32_fast": 4}
 
 
 def rys_roots(T, nroots: int, fp32: bool = False, device: int = 0, path: Optional[str] = None):
     """Device Rys roots and weights; ``path`` selects one of the kernels'
-    evaluation paths (RYS_PATHS), default the FP64 (or FP32) tables."""
+    evaluation paths (RYS_PATHS): "fp64_table" / "fp32_table" (default) is the
+    root-by-root lookup of the block- and warp-per-quartet kernels, "fp64_fast"
+    / "fp32_fast" what the compile-time kernels run (nroots <= 5)."""
     T = _f64(np.atleast_1d(T))
     r = np.empty((len(T), nroots))
     w = np.empty((len(T), nroots))
