@@ -278,6 +278,9 @@ int tlno_gpu_boys(int device, int n, int maxn, const double* x, double* out);
  * in their FP32 pass (nroots <= 5; a NaN argument is passed on to them). */
 int tlno_gpu_rys(int device, int n, int nroots, const double* T, double* roots, double* weights,
                  int fp32);
+/* 1/sqrt(x) as the ERI kernels evaluate it, at n positive normal arguments
+ * (host buffers): mode 0 FP64, 1 FP32. */
+int tlno_gpu_rsqrt(int device, int n, const double* x, double* out, int mode);
 
 /* Measured FP64 FMA throughput of the device (TFLOP/s, 2 flops per FMA)
  * from a dependent-chain DFMA kernel filling every SM; the roofline

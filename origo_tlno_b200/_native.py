@@ -115,6 +115,7 @@ def lib() -> C.CDLL:
         "tlno_gpu_schwarz": (C.c_int, [_vp, _vp]),
         "tlno_gpu_boys": (C.c_int, [C.c_int, C.c_int, C.c_int, _vp, _vp]),
         "tlno_gpu_rys": (C.c_int, [C.c_int, C.c_int, C.c_int, _vp, _vp, _vp, C.c_int]),
+        "tlno_gpu_rsqrt": (C.c_int, [C.c_int, C.c_int, _vp, _vp, C.c_int]),
         "tlno_gpu_fma_peak": (C.c_int, [C.c_int, C.c_int, _dp]),
         "tlno_gpu_jk_graph_capture": (C.c_int, [_vp, _vp, _vp, _vp, C.c_int]),
         "tlno_gpu_jk_graph_launch": (C.c_int, [_vp]),
@@ -170,7 +171,7 @@ EXPORTED = [
     "tlno_gpu_incremental_reset", "tlno_gpu_incremental_fail_next_update",
     "tlno_gpu_onee", "tlno_gpu_set_onee_thresholds",
     "tlno_gpu_set_mixed_threshold",
-    "tlno_gpu_eri_blocks", "tlno_gpu_eri_blocks_noalloc", "tlno_gpu_schwarz", "tlno_gpu_boys", "tlno_gpu_rys", "tlno_gpu_fma_peak",
+    "tlno_gpu_eri_blocks", "tlno_gpu_eri_blocks_noalloc", "tlno_gpu_schwarz", "tlno_gpu_boys", "tlno_gpu_rys", "tlno_gpu_rsqrt", "tlno_gpu_fma_peak",
     "tlno_gpu_jk_graph_capture",
     "tlno_gpu_jk_graph_launch", "tlno_gpu_synchronize", "tlno_gpu_stream", "tlno_gpu_batch_create",
     "tlno_gpu_batch_destroy", "tlno_gpu_batch_total_elements", "tlno_gpu_batch_offsets",

@@ -226,6 +226,13 @@ __global__ void rys_fast_test_kernel(const double* T, int n, int mode, double* r
     }
 }
 
+// Test hook of rsqrt_pos.
+template <typename R>
+__global__ void rsqrt_test_kernel(const double* x, int n, double* out) {
+    const int i = blockIdx.x * blockDim.x + threadIdx.x;
+    if (i < n) out[i] = double(rsqrt_pos(R(x[i])));
+}
+
 __global__ void absmax_kernel(const double* x, long long n, double* out) {
     __shared__ double red[32];
     double m = 0.0;
@@ -786,6 +793,14 @@ double measure_fma_peak(bool fp32) {
 
 void launch_boys_test(const double* x, int n, int maxn, double* out, cudaStream_t s) {
     boys_test_kernel<<<(n + 127) / 128, 128, 0, s>>>(x, n, maxn, out);
+    TLNO_CUDA(cudaGetLastError());
+}
+
+void launch_rsqrt_test(const double* x, int n, int mode, double* out, cudaStream_t s) {
+    if (mode == 1)
+        rsqrt_test_kernel<float><<<(n + 127) / 128, 128, 0, s>>>(x, n, out);
+    else
+        rsqrt_test_kernel<double><<<(n + 127) / 128, 128, 0, s>>>(x, n, out);
     TLNO_CUDA(cudaGetLastError());
 }
 

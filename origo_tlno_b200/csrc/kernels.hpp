@@ -94,6 +94,8 @@ void launch_combine_g(const double* J, const double* K, double* G, long long n, 
 // Dependent-chain FMA throughput probe: returns TFLOP/s.
 double measure_fma_peak(bool fp32);
 void launch_boys_test(const double* x, int n, int maxn, double* out, cudaStream_t s);
+// rsqrt_pos of the ERI kernels at n arguments, FP64 (mode 0) or FP32 (mode 1).
+void launch_rsqrt_test(const double* x, int n, int mode, double* out, cudaStream_t s);
 void launch_rys_test(const double* t, int n, int nroots, int fp32, double* roots, double* weights,
                      cudaStream_t s);
 

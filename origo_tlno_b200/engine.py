@@ -524,3 +524,11 @@ def rys_roots(T, nroots: int, fp32: bool = False, device: int = 0, path: Optiona
     mode = RYS_PATHS[path] if path else (1 if fp32 else 0)
     N.check(N.lib().tlno_gpu_rys(device, len(T), nroots, N.ptr(T), N.ptr(r), N.ptr(w), mode))
     return r, w
+
+
+def rsqrt(x, fp32: bool = False, device: int = 0) -> np.ndarray:
+    """1/sqrt(x) of positive normal arguments as the ERI kernels evaluate it."""
+    x = _f64(np.atleast_1d(x))
+    out = np.empty(len(x))
+    N.check(N.lib().tlno_gpu_rsqrt(device, len(x), N.ptr(x), N.ptr(out), 1 if fp32 else 0))
+    return out
