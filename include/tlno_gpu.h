@@ -279,7 +279,8 @@ int tlno_gpu_boys(int device, int n, int maxn, const double* x, double* out);
 int tlno_gpu_rys(int device, int n, int nroots, const double* T, double* roots, double* weights,
                  int fp32);
 /* 1/sqrt(x) as the ERI kernels evaluate it, at n positive normal arguments
- * (host buffers): mode 0 FP64, 1 FP32. */
+ * (host buffers): mode 0 FP64, 1 FP32 of the compile-time kernels; 2 FP64,
+ * 3 FP32 of the block-per-quartet row kernel, 1/x and 1/sqrt(x) interleaved. */
 int tlno_gpu_rsqrt(int device, int n, const double* x, double* out, int mode);
 
 /* Measured FP64 FMA throughput of the device (TFLOP/s, 2 flops per FMA)

@@ -869,16 +869,18 @@ int tlno_gpu_rys(int device, int n, int nroots, const double* T, double* roots, 
 
 int tlno_gpu_rsqrt(int device, int n, const double* x, double* out, int mode) {
     return guarded([&] {
-        if (n < 0 || mode < 0 || mode > 1 || (n > 0 && (!x || !out)))
+        if (n < 0 || mode < 0 || mode > 3 || (n > 0 && (!x || !out)))
             throw Error(TLNO_GPU_E_INVALID, "tlno_gpu: bad reciprocal square root arguments");
         set_device(device);
         if (n == 0) return;
         DeviceBuffer dx, dout;
         dx.alloc(sizeof(double) * n);
-        dout.alloc(sizeof(double) * n);
+        const std::size_t bytes = sizeof(double) * n * (mode >= 2 ? 2 : 1);
+        dout.alloc(bytes);
         TLNO_CUDA(cudaMemcpy(dx.ptr, x, sizeof(double) * n, cudaMemcpyHostToDevice));
-        launch_rsqrt_test(dx.as<double>(), n, mode, dout.as<double>(), 0);
-        TLNO_CUDA(cudaMemcpy(out, dout.ptr, sizeof(double) * n, cudaMemcpyDeviceToHost));
+        if (mode >= 2) launch_reciprocals_test(dx.as<double>(), n, mode == 3, dout.as<double>(), 0);
+        else launch_rsqrt_test(dx.as<double>(), n, mode, dout.as<double>(), 0);
+        TLNO_CUDA(cudaMemcpy(out, dout.ptr, bytes, cudaMemcpyDeviceToHost));
     });
 }
 

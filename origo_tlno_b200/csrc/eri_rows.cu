@@ -26,6 +26,17 @@ void rows_upload(const dev::DevTables& t, const dev::CartTable& c, const dev::C2
 
 namespace {
 
+// Test hook of reciprocals: out[2 i] = 1/x, out[2 i + 1] = 1/sqrt(x).
+template <typename R>
+__global__ void reciprocals_test_kernel(const double* x, int n, double* out) {
+    const int i = blockIdx.x * blockDim.x + threadIdx.x;
+    if (i >= n) return;
+    R inv, rs;
+    dev::reciprocals(R(x[i]), inv, rs);
+    out[2 * i] = double(inv);
+    out[2 * i + 1] = double(rs);
+}
+
 template <typename R, int LC, int LD>
 void launch(const dev::PlanView& pv, const dev::ClassLaunch& cl, int sms, cudaStream_t s) {
     // item slots per batch: 32 (64 take the shared memory of resident blocks),
@@ -50,6 +61,12 @@ void launch(const dev::PlanView& pv, const dev::ClassLaunch& cl, int sms, cudaSt
 }
 
 }  // namespace
+
+void launch_reciprocals_test(const double* x, int n, bool fp32, double* out, cudaStream_t s) {
+    if (fp32) reciprocals_test_kernel<float><<<(n + 127) / 128, 128, 0, s>>>(x, n, out);
+    else reciprocals_test_kernel<double><<<(n + 127) / 128, 128, 0, s>>>(x, n, out);
+    TLNO_CUDA(cudaGetLastError());
+}
 
 bool launch_eri_jk_rows(const dev::PlanView& pv, const dev::ClassLaunch& cl, bool fp32, int sms, cudaStream_t s) {
     if (cl.la > 3 || cl.la + cl.lb < 2) return false;

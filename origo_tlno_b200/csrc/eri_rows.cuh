@@ -80,6 +80,17 @@ struct RowsLayout {
     }
 };
 
+// 1/x and 1/sqrt(x) of p + q, each within the rounding of a division and a
+// square root: rsqrt_pos (in FP32, the bare instruction of 2^-22.9, one Newton
+// step further) and one step on its square.
+template <typename R>
+__device__ __forceinline__ void reciprocals(R x, R& inv, R& rs) {
+    rs = rsqrt_pos(x);
+    if (sizeof(R) == 4) rs = fma(R(0.5) * rs, fma(-x * rs, rs, R(1)), rs);
+    inv = rs * rs;
+    inv = fma(inv, fma(-x, inv, R(1)), inv);
+}
+
 // One axis table in registers, column by column:
 // G(i, k+1) = d00 G(i, k) + i b00 G(i-1, k) + k b01 G(i, k-1).
 template <typename R, int LAB, int LCD, int KSP>
@@ -207,8 +218,8 @@ __device__ void rows_quartet(const PlanView& pv, const ClassLaunch& cl, const Ro
             const DPrimPair bp = pb[ib];
             const DPrimPair kp = pk[ik];
             const R p = R(bp.p), q = R(kp.p);
-            const R rs = rsqrt_pos(p + q);
-            const R inv = rs * rs;
+            R inv, rs;
+            reciprocals(p + q, inv, rs);
             const R PQ[3] = {R(bp.Px) - R(kp.Px), R(bp.Py) - R(kp.Py), R(bp.Pz) - R(kp.Pz)};
             const R Targ = p * q * inv * (PQ[0] * PQ[0] + PQ[1] * PQ[1] + PQ[2] * PQ[2]);
             R t2, wt;

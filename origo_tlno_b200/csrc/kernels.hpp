@@ -48,6 +48,8 @@ inline int block_tile_part(long long ntiles, int bk, int wave) {
 // class it does not cover.
 void rows_upload(const dev::DevTables& t, const dev::CartTable& c, const dev::C2STable& s);
 bool launch_eri_jk_rows(const dev::PlanView& pv, const dev::ClassLaunch& cl, bool fp32, int sms, cudaStream_t s);
+// The row kernel's 1/x and 1/sqrt(x), interleaved, at n arguments.
+void launch_reciprocals_test(const double* x, int n, bool fp32, double* out, cudaStream_t s);
 // Pair records of a plan (view with its pair and shell arrays filled).
 void launch_pair_records(const dev::PlanView& pv, int n_pairs, dev::PairRec* out, cudaStream_t s);
 bool has_fast_kernel(int la, int lb, int lc, int ld);

@@ -532,3 +532,11 @@ def rsqrt(x, fp32: bool = False, device: int = 0) -> np.ndarray:
     out = np.empty(len(x))
     N.check(N.lib().tlno_gpu_rsqrt(device, len(x), N.ptr(x), N.ptr(out), 1 if fp32 else 0))
     return out
+
+
+def reciprocals(x, fp32: bool = False, device: int = 0):
+    """(1/x, 1/sqrt(x)) as the row kernel evaluates them."""
+    x = _f64(np.atleast_1d(x))
+    out = np.empty((len(x), 2))
+    N.check(N.lib().tlno_gpu_rsqrt(device, len(x), N.ptr(x), N.ptr(out), 3 if fp32 else 2))
+    return out[:, 0], out[:, 1]

@@ -113,3 +113,21 @@ def test_reciprocal_square_root():
     err32 = float(np.max(np.abs(E.rsqrt(x32, fp32=True) / exact - 1)))
     print(f"PIN rsqrt fp64={err:.3e} fp32={err32:.3e}")
     assert err < 1.67e-16 and err32 < 2.0 ** -22.9
+
+
+@pytest.mark.parametrize("fp32", [False, True])
+def test_row_kernel_reciprocals(fp32):
+    # as accurate as a division and a square root: 1/x to one rounding of its
+    # Newton step (u, and a second-order rest below u/16), 1/sqrt(x) to u plus
+    # half a rounding of the residual, u = 2^-53 or 2^-24
+    rng = np.random.default_rng(4)
+    x = np.exp(rng.uniform(np.log(1e-6), np.log(1e12), 200000))
+    if fp32:
+        x = x.astype(np.float32)
+    inv, rs = E.reciprocals(x, fp32=fp32)
+    xl = x.astype(np.longdouble)
+    u = 2.0 ** -24 if fp32 else 2.0 ** -53
+    e_inv = float(np.max(np.abs(inv * xl - 1)))
+    e_rs = float(np.max(np.abs(rs * np.sqrt(xl) - 1)))
+    print(f"PIN reciprocals {'fp32' if fp32 else 'fp64'} inv={e_inv / u:.3f} u rs={e_rs / u:.3f} u")
+    assert e_inv <= 1.0625 * u and e_rs <= 1.5625 * u
