@@ -318,10 +318,11 @@ int tlno_gpu_batch_synchronize(tlno_gpu_batch* b);
 void* tlno_gpu_batch_stream(tlno_gpu_batch* b);
 
 /* Tuning of the kernel schedule: generic-kernel ket tile, generic warps
- * per CTA (0 = the block-per-quartet generic kernel with the plan's pair
- * projectors, or, for a plan too large to keep them, the warp-per-quartet
- * kernel with warps from the shared-memory budget; 1..8 = the
- * warp-per-quartet kernel with that many warps), persistent grid multiplier
+ * per CTA of the classes without a compile-time kernel (0 = the
+ * block-per-quartet kernel with the plan's pair projectors, or, for pair
+ * classes too large to keep them, the warp-per-quartet kernel with warps from
+ * the shared-memory budget; 1..8 = the warp-per-quartet kernel with that many
+ * warps; (dd|dd), (dd|dp) and (fp|dp) keep the block kernel where they have it), persistent grid multiplier
  * (the compile-time kernels size their grid from the occupancy calculator,
  * capped by grid_mult x SMs), and streams (1..4): the class launches of a
  * build spread over that many streams (parallel branches of a captured
@@ -338,6 +339,11 @@ typedef struct {
 int tlno_gpu_set_tuning(tlno_gpu_context* ctx, const tlno_gpu_tuning* t);
 /* The same for a batch (its schedule keeps the ket tile of its plan). */
 int tlno_gpu_batch_set_tuning(tlno_gpu_batch* b, const tlno_gpu_tuning* t);
+/* Device memory that the next plan of the context may spend on pair-projector
+ * tables (default 16 GB): the pair classes with the smallest tables get them
+ * while they fit, and a class combination of which one has none runs the
+ * warp-per-quartet kernel. */
+int tlno_gpu_set_projector_limit(tlno_gpu_context* ctx, long long bytes);
 int tlno_gpu_set_combo_generic(tlno_gpu_context* ctx, int combo_id, int force_generic);
 /* Per class-combination statistics of the current plan: for i < n, writes
  * (X, Y, la, lb, lc, ld, fast, n_tiles) into ints[8*i] and

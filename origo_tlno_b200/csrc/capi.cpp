@@ -295,7 +295,7 @@ void enqueue_jk(Plan2e& plan, const Tuning& tune, const BuildSpec& spec, const d
         if (cs.fast)
             launch_eri_jk_fast(pv, cl, fp32, grid, cs_stream);
         else
-            launch_eri_jk_generic(pv, cl, fp32, tune.generic_warps, grid, cs_stream);
+            launch_eri_jk_generic(pv, cl, fp32, cs.generic_form(tune), grid, cs_stream);
     }
     branches.join();
     if (plan.n_mol > 1) {
@@ -619,7 +619,7 @@ int tlno_gpu_eri_checksum(tlno_gpu_context* ctx, double* checksum, double* ms) {
             if (cs.fast)
                 launch_eri_jk_fast(pv, cl, false, grid, s);
             else
-                launch_eri_jk_generic(pv, cl, false, ctx->tune.generic_warps, grid, s);
+                launch_eri_jk_generic(pv, cl, false, cs.generic_form(ctx->tune), grid, s);
         }
         TLNO_CUDA(cudaEventRecord(e1, s));
         TLNO_CUDA(cudaMemcpyAsync(checksum, d_sum, sizeof(double), cudaMemcpyDeviceToHost, s));
@@ -960,6 +960,13 @@ int tlno_gpu_set_tuning(tlno_gpu_context* ctx, const tlno_gpu_tuning* t) {
     });
 }
 
+int tlno_gpu_set_projector_limit(tlno_gpu_context* ctx, long long bytes) {
+    return guarded([&] {
+        if (!ctx || bytes < 0) throw Error(TLNO_GPU_E_INVALID, "tlno_gpu: projector limit must be >= 0");
+        ctx->tune.max_projector_bytes = bytes;
+    });
+}
+
 int tlno_gpu_set_combo_generic(tlno_gpu_context* ctx, int combo_id, int force_generic) {
     return guarded([&] {
         if (!ctx || combo_id < 0 || combo_id >= 256) throw Error(TLNO_GPU_E_INVALID, "tlno_gpu: bad combo id");
@@ -1030,7 +1037,7 @@ int tlno_gpu_time_combo(tlno_gpu_context* ctx, int combo_index, int mode, int re
         auto run = [&] {
             TLNO_CUDA(cudaMemsetAsync(cl.counter, 0, sizeof(int), s));
             if (cs.fast) launch_eri_jk_fast(pv, cl, fp32 != 0, grid, s);
-            else launch_eri_jk_generic(pv, cl, fp32 != 0, ctx->tune.generic_warps, grid, s);
+            else launch_eri_jk_generic(pv, cl, fp32 != 0, cs.generic_form(ctx->tune), grid, s);
         };
         run();
         TLNO_CUDA(cudaEventRecord(e0, s));
@@ -1116,7 +1123,7 @@ int tlno_gpu_class_jk(tlno_gpu_context* ctx, int combo_index, const double* d_de
             if (cs.fast)
                 launch_eri_jk_fast(pv, cl, fp32, sms * ctx->tune.grid_mult, s);
             else
-                launch_eri_jk_generic(pv, cl, fp32, ctx->tune.generic_warps, sms * ctx->tune.grid_mult, s);
+                launch_eri_jk_generic(pv, cl, fp32, cs.generic_form(ctx->tune), sms * ctx->tune.grid_mult, s);
         }
         TLNO_CUDA(cudaEventRecord(e1, s));
         TLNO_CUDA(cudaEventSynchronize(e1));

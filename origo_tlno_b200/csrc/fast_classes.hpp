@@ -2,12 +2,9 @@
 // index >= ket class index): every class with shells up to d except (dd|dd)
 // and the f classes with one f shell whose instantiation compiles in a few
 // minutes (bra (fs), (fp) against kets up to (dp)/(fs), (fd) against (ss),
-// (ps), (ds)).  The other classes take the block-per-quartet kernel
-// (eri_rows.cuh); (dd|dd), 8 slices of spilled registers here, runs there in
-// 0.53 instead of 1.01 ms (f-shell 14 atoms), 0.098 / 0.094 ms (24-atom
-// organic), 0.61 / 0.54 ms of 290 (91 waters).  (dd|dp), (fp|dp), (fp|pp) gain
-// there only with deep contractions (3.7 / 4.7, 4.0 / 4.7, 2.9 / 2.8 ms, but
-// 16.8 / 5.2 ms for (dd|dp) of 91 waters) and stay.  Each class
+// (ps), (ds)).  The other classes take the block-per-quartet kernel (eri_rows.cuh);
+// so do (dd|dp) and (fp|dp) where their contraction is deep (the rule and the
+// figures of all three: block_kernel_class in plan.cpp).  Each class
 // is compiled in its own translation unit (eri_fast_inst.cu with
 // -DTLNO_FAST_ID=<index>).
 #pragma once

@@ -576,7 +576,8 @@ static void generic_cta_shape(int la, int lb, int lc, int ld, int& threads, int&
 void launch_eri_jk_generic(const PlanView& pv, const ClassLaunch& cl, bool fp32, int warps, int grid,
                            cudaStream_t s) {
     if (cl.tile_end <= cl.tile_begin) return;
-    if (pv.proj && warps <= 0) {
+    if (warps == 0) {
+        if (!pv.proj) throw Error(-3, "tlno_gpu: block-per-quartet launch without projectors");
         if (launch_eri_jk_rows(pv, cl, fp32, sm_count(), s)) return;
         // one quartet per block at a time, projectors from the plan
         int threads = 0, nb_items = 0, bytes = 0;

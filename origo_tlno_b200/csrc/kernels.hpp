@@ -27,6 +27,9 @@ void launch_pair_projectors(const int* pair_A, const int* pair_B, const double* 
 
 void launch_eri_store(const dev::PlanView& pv, const dev::ClassLaunch& cl, cudaStream_t s);
 void launch_eri_schwarz(const dev::PlanView& pv, const dev::ClassLaunch& cl, cudaStream_t s);
+// J/K launch of a class without a compile-time kernel: warps 0 = block per
+// quartet (needs the plan's projectors), > 0 = warp per quartet with that many
+// warps per block, < 0 = with warps from the shared-memory budget.
 void launch_eri_jk_generic(const dev::PlanView& pv, const dev::ClassLaunch& cl, bool fp32,
                            int warps, int grid, cudaStream_t s);
 // Thread-per-quartet kernels for the classes that have one; returns false

@@ -110,14 +110,27 @@ double flops_per_prim(int a, int b, int c, int d) {
 }
 // Classes with a compile-time kernel of 4 register slices that the
 // block-per-quartet kernel beats where the contraction is deep, that is where
-// the primitive loop outweighs its barriers: (dd|dp) 2.0 | 4.8 ms at 8.4
-// primitive quartets per quartet (f-shell 14 atoms), 8.5 | 5.2 ms at 1.2 (91
-// waters); (fp|dp) 2.5 | 4.7 ms at 11.7.  The projectors this needs (2-6 KB per
-// pair) are affordable up to a million pairs.
+// the primitive loop outweighs its barriers, block | compile-time: (dd|dp) 2.0 |
+// 4.7 ms at 8.4 primitive quartets per quartet (f-shell 14 atoms), 0.41 | 0.33 at
+// 1.8 (24-atom organic), 7.8 | 5.2 at 1.2 (91 waters); (fp|dp) 2.5 | 4.6 at 11.7.
+// The projectors this needs (2-6 KB per pair) are affordable up to a million
+// pairs, and only while the tables of the classes that have no other fast
+// kernel fit beside them; the kernel's item index (primitive quartets x roots)
+// has to fit 31 bits.
 constexpr double kBlockKernelPrims = 4.0;
 constexpr long long kBlockKernelPairs = 1000000;
 bool block_kernel_class(int la, int lb, int lc, int ld) {
     return lc == 2 && ld == 1 && ((la == 2 && lb == 2) || (la == 3 && lb == 1));
+}
+// (dd|dd) has no compile-time kernel (8 slices of spilled registers): block |
+// compile-time FP64 0.45 | 0.92 ms (f-shell 14 atoms), 0.083 | 0.086 (24-atom
+// organic), 0.53 | 0.55 (91 waters), FP32 0.43 | 0.68, 0.083 | 0.063, 0.53 | 0.39.
+bool block_only_class(int la, int lb, int lc, int ld) { return la == 2 && lb == 2 && lc == 2 && ld == 2; }
+
+// Projector words of one pair (HRR + spherical map, eri_generic.cuh).
+long long projector_words(int la, int lb) {
+    const int nslice = (la + lb + 1) * (la + lb + 2) * (la + lb + 3) / 6 - la * (la + 1) * (la + 2) / 6;
+    return static_cast<long long>(2 * la + 1) * (2 * lb + 1) * nslice;
 }
 
 // ---- tile shapes of the compile-time kernels ----
@@ -578,16 +591,21 @@ void build_plan(Plan2e& plan, const std::vector<const Basis*>& bases, std::vecto
     plan.combos.clear();
     plan.total_quartets = plan.total_prim_quartets = 0;
     plan.total_flops = 0.0;
-    // Mean primitive count of a pair class.
-    auto mean_nprim = [&](int X) {
-        double n = 0.0, sum = 0.0;
-        for (int m = 0; m < plan.n_mol; ++m)
-            for (int k = 0; k < plan.mol_pairs[m].cls_count[X]; ++k) {
-                sum += plan.pair_nprim[gbeg[m][X] + k];
-                n += 1.0;
-            }
-        return n > 0.0 ? sum / n : 0.0;
+    // Per pair class: kept pairs, mean and largest primitive count.
+    struct ClassPrims {
+        long long n = 0, sum = 0;
+        int max = 0;
+        double mean() const { return n > 0 ? double(sum) / n : 0.0; }
     };
+    std::array<ClassPrims, kMaxPairClasses> prims{};
+    for (int m = 0; m < plan.n_mol; ++m)
+        for (int X = 0; X < kMaxPairClasses; ++X)
+            for (int k = 0; k < plan.mol_pairs[m].cls_count[X]; ++k) {
+                const int np = plan.pair_nprim[gbeg[m][X] + k];
+                prims[X].n += 1;
+                prims[X].sum += np;
+                prims[X].max = std::max(prims[X].max, np);
+            }
     // The class schedules are independent: built on host threads, uploaded in
     // class order.
     std::vector<ComboSchedule> todo;
@@ -609,16 +627,52 @@ void build_plan(Plan2e& plan, const std::vector<const Basis*>& bases, std::vecto
             cs.lc = lc; cs.ld = Y - lc * (lc + 1) / 2;
             const int combo_id = X * kMaxPairClasses + Y;
             cs.fast = has_fast_kernel(cs.la, cs.lb, cs.lc, cs.ld) &&
-                      !(combo_id < 256 && tune.force_generic[combo_id]) &&
-                      !(block_kernel_class(cs.la, cs.lb, cs.lc, cs.ld) &&
-                        mean_nprim(X) * mean_nprim(Y) >= kBlockKernelPrims && plan.kept_pairs <= kBlockKernelPairs);
-            cs.bb = cs.fast ? fast_kernel_bras(cs.la, cs.lb, cs.lc, cs.ld) : 1;
-            cs.bk = cs.fast ? 32 : tune.generic_bk;
+                      !(combo_id < 256 && tune.force_generic[combo_id]);
+            cs.block = block_only_class(cs.la, cs.lb, cs.lc, cs.ld);
             todo.push_back(std::move(cs));
-            resident.push_back(todo.back().fast ? fast_kernel_resident_groups(todo.back().la, todo.back().lb,
-                                                                              todo.back().lc, todo.back().ld)
-                                                : 1);
         }
+    // Projector tables: those of the classes without a compile-time kernel, the
+    // smallest first while they fit, then those of the classes with a choice.
+    std::array<bool, kMaxPairClasses> table{};
+    {
+        std::array<long long, kMaxPairClasses> bytes{};
+        std::array<bool, kMaxPairClasses> wanted{};
+        for (const ComboSchedule& cs : todo) {
+            bytes[cs.X] = 8 * prims[cs.X].n * projector_words(cs.la, cs.lb);
+            bytes[cs.Y] = 8 * prims[cs.Y].n * projector_words(cs.lc, cs.ld);
+            if (!cs.fast) wanted[cs.X] = wanted[cs.Y] = true;
+        }
+        std::vector<int> order;
+        for (int X = 0; X < kMaxPairClasses; ++X)
+            if (wanted[X]) order.push_back(X);
+        std::stable_sort(order.begin(), order.end(), [&](int a, int b) { return bytes[a] < bytes[b]; });
+        long long left = tune.max_projector_bytes;
+        bool all = true;
+        for (int X : order) {
+            all = all && bytes[X] <= left;
+            if (!all) break;
+            left -= bytes[X];
+            table[X] = true;
+        }
+        for (ComboSchedule& cs : todo) {
+            if (!all || !cs.fast || !block_kernel_class(cs.la, cs.lb, cs.lc, cs.ld) || tune.generic_warps > 0) continue;
+            const int nroots = (cs.la + cs.lb + cs.lc + cs.ld) / 2 + 1;
+            const long long more = (table[cs.X] ? 0 : bytes[cs.X]) + (table[cs.Y] ? 0 : bytes[cs.Y]);
+            if (prims[cs.X].mean() * prims[cs.Y].mean() < kBlockKernelPrims || plan.kept_pairs > kBlockKernelPairs ||
+                double(prims[cs.X].max) * prims[cs.Y].max * nroots > 2147483647.0 || more > left)
+                continue;
+            left -= more;
+            table[cs.X] = table[cs.Y] = true;
+            cs.fast = false;
+            cs.block = true;
+        }
+    }
+    for (ComboSchedule& cs : todo) {
+        cs.proj = !cs.fast && table[cs.X] && table[cs.Y];
+        cs.bb = cs.fast ? fast_kernel_bras(cs.la, cs.lb, cs.lc, cs.ld) : 1;
+        cs.bk = cs.fast ? 32 : tune.generic_bk;
+        resident.push_back(cs.fast ? fast_kernel_resident_groups(cs.la, cs.lb, cs.lc, cs.ld) : 1);
+    }
     auto build_schedule = [&](ComboSchedule& cs, int resident_groups) {
         const int X = cs.X, Y = cs.Y;
         const double fprim = flops_per_prim(cs.la, cs.lb, cs.lc, cs.ld);
@@ -795,12 +849,12 @@ void build_plan(Plan2e& plan, const std::vector<const Basis*>& bases, std::vecto
     }
     plan.d_counters.alloc(sizeof(int) * 2 * std::max<std::size_t>(plan.combos.size(), 1));
 
-    // HRR + spherical projectors of the pairs of every pair class that a
-    // generic (CTA) class combination uses, built once on the device.
+    // HRR + spherical projectors of the pairs of the classes that a
+    // block-per-quartet combination uses, built once on the device.
     {
         std::array<bool, kMaxPairClasses> need{};
         for (const ComboSchedule& cs : plan.combos)
-            if (!cs.fast) need[cs.X] = need[cs.Y] = true;
+            if (cs.proj) need[cs.X] = need[cs.Y] = true;
         const std::size_t np = plan.pair_A.size();
         plan.proj_off.assign(np, -1);
         long long words = 0;
@@ -808,13 +862,21 @@ void build_plan(Plan2e& plan, const std::vector<const Basis*>& bases, std::vecto
             const int la = Ls[plan.pair_A[k]], lb = Ls[plan.pair_B[k]];
             if (!need[la * (la + 1) / 2 + lb]) continue;
             plan.proj_off[k] = words;
-            const int nslice = (la + lb + 1) * (la + lb + 2) * (la + lb + 3) / 6 - la * (la + 1) * (la + 2) / 6;
-            words += static_cast<long long>(2 * la + 1) * (2 * lb + 1) * nslice;
+            words += projector_words(la, lb);
         }
         plan.proj_words = words;
         plan.proj_ready = false;
-        if (words > 0 && words * 8 <= kMaxProjectorBytes) {
-            plan.d_proj.alloc(sizeof(double) * words);
+        if (words > 0) {
+            try {
+                plan.d_proj.alloc(sizeof(double) * words);
+            } catch (const Error&) {
+                // no room on the device: the classes run warp per quartet
+                cudaGetLastError();
+                for (ComboSchedule& cs : plan.combos) cs.proj = false;
+                words = 0;
+            }
+        }
+        if (words > 0) {
             upload_vec(plan.d_proj_off, plan.proj_off, s);
             launch_pair_projectors(plan.d_pair_A.as<int>(), plan.d_pair_B.as<int>(), plan.d_shell_xyz.as<double>(),
                                    plan.d_shell_L.as<int>(), plan.d_proj_off.as<long long>(), static_cast<int>(np),

@@ -11,9 +11,11 @@
 
 namespace tlno_gpu {
 
-// Largest pair-projector table a plan keeps on the device; above it the
-// generic classes run the warp-per-quartet kernel, which builds projectors
-// per quartet.
+// Device memory a plan may spend on pair-projector tables.  A table saves the
+// block-per-quartet kernels the maps of every quartet (f-shell 14 atoms, the 18
+// classes without a compile-time kernel: 12.9 ms with it, 160 ms in the
+// warp-per-quartet kernel, which builds them per quartet), so it may take up to
+// a tenth of the device.
 constexpr long long kMaxProjectorBytes = 16LL << 30;
 
 struct Tuning {
@@ -21,6 +23,7 @@ struct Tuning {
     int generic_warps = 0;  // 0 = from shared-memory budget
     int grid_mult = 8;      // CTAs per SM for persistent launches
     int streams = 0;        // streams the class launches of a build spread over (0 = by the plan's size)
+    long long max_projector_bytes = kMaxProjectorBytes;
     std::array<int, 256> force_generic{};  // per class combo: 1 = never use the fast kernel
 };
 
@@ -28,11 +31,21 @@ struct ComboSchedule {
     int X = 0, Y = 0;            // pair classes, X >= Y
     int la = 0, lb = 0, lc = 0, ld = 0;
     bool fast = false;
+    bool proj = false;   // both pair classes have projector tables: block-per-quartet kernel
+    bool block = false;  // the block-per-quartet kernel took over from a compile-time one
+                         // (block_kernel_class in plan.cpp): generic_warps does not apply
     int bb = 1, bk = 16;
     // per-class tuning: split threshold multiplier of the mixed path and
     // tiles per dynamic-schedule fetch (0 = kernel default)
     double mix_scale = 1.0;
     int chunk = 0;
+    // launch form of a class without a compile-time kernel: 0 = block per
+    // quartet, > 0 = warp per quartet with that many warps, < 0 = with warps
+    // from the shared-memory budget
+    int generic_form(const Tuning& t) const {
+        if (!proj) return t.generic_warps > 0 ? t.generic_warps : -1;
+        return block ? 0 : t.generic_warps;
+    }
     std::vector<dev::BlockDesc> blocks;
     std::vector<int> prefix;
     std::vector<int> bra_list;
@@ -82,7 +95,8 @@ public:
     // heuristic decay indicator (integral_threshold must then be 0).
     bool decay_metric = false;
     // Pair projectors (HRR + spherical maps) of the pair classes the generic
-    // class combinations use: per pair its offset into d_proj or -1.
+    // class combinations use, the smallest tables first while they fit
+    // Tuning::max_projector_bytes: per pair its offset into d_proj or -1.
     std::vector<long long> proj_off;
     DeviceBuffer d_proj, d_proj_off;
     long long proj_words = 0;

@@ -232,6 +232,10 @@ class Context:
         t = N.Tuning(generic_bk, generic_warps, grid_mult, streams)
         N.check(N.lib().tlno_gpu_set_tuning(self.h, C.byref(t)))
 
+    def set_projector_limit(self, nbytes: int):
+        """Device memory the next plan may spend on pair-projector tables."""
+        N.check(N.lib().tlno_gpu_set_projector_limit(self.h, nbytes))
+
     def set_combo_generic(self, combo_id: int, force: bool):
         N.check(N.lib().tlno_gpu_set_combo_generic(self.h, combo_id, 1 if force else 0))
 

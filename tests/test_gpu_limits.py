@@ -22,3 +22,34 @@ def test_batch_refuses_more_functions_than_the_matrix_indices_hold():
         E.Batch([small, big])
     big.close()
     small.close()
+
+
+def test_projector_limit_and_warp_form_give_the_same_matrices():
+    # with less memory than the projector tables need the largest go first; the
+    # classes without one run warp per quartet, (dd|dp) and (fp|dp) then keep
+    # their compile-time kernels, and a warp form asked for leaves the classes
+    # the block kernel took over from a compile-time one where they are
+    mol = M.fragment(M.cfg2(), [0, 1, 2])
+    D = M.random_density(mol.n_sph, max(1, mol.n_sph // 5), seed=3)
+    opts = E.ScreeningOptions(integral_threshold=1e-12)
+    ctx = E.Context(mol).plan(opts)
+    ref, mixed = ctx.jk(D), ctx.jk(D, mixed=True)
+    n_fast = sum(c["fast"] for c in ctx.combos())
+    for limit in (0, 20000, 400000, 4000000, 1 << 34):
+        ctx.set_projector_limit(limit)
+        ctx.plan(opts)
+        assert sum(c["fast"] for c in ctx.combos()) >= n_fast
+        out, out32 = ctx.jk(D), ctx.jk(D, mixed=True)
+        for k in ("J", "K"):
+            assert np.max(np.abs(out[k] - ref[k])) < 1e-12
+            assert np.max(np.abs(out32[k] - mixed[k])) < 1e-7
+    for warps in (1, 4):
+        ctx.set_tuning(generic_warps=warps)
+        for replan in (False, True):
+            if replan:
+                ctx.plan(opts)
+            out = ctx.jk(D)
+            assert max(np.max(np.abs(out[k] - ref[k])) for k in ("J", "K")) < 1e-12
+    with pytest.raises(E.TlnoError, match="limit"):
+        ctx.set_projector_limit(-1)
+    ctx.close()
