@@ -402,7 +402,7 @@ def run_batch(args):
     opts = E.ScreeningOptions(integral_threshold=1e-12, mixed_threshold=args.mixed_threshold)
     ctxs = [E.Context(m, device=local) for m in mols]
     batch = E.Batch(ctxs, opts)
-    if args.streams > 1:
+    if args.streams > 0:
         batch.set_tuning(streams=args.streams)
     prof = batch.profile()
     Ds = [torch.tensor(MOL.random_density(m.n_sph, max(1, m.n_sph // 5), seed=100 + i)) for i, m in enumerate(mols)]
@@ -492,7 +492,7 @@ def run_batch(args):
            "config": {"workload": "cfg3", "description": "256 molecules of 3-30 atoms in one batch, Schwarz 1e-12",
                       "l2": "L2 flushed between timed builds (256 MB write)",
                       "molecules": len(mols), "functions_total": prof["M"], "quartets_per_build": q,
-                      "streams": args.streams},
+                      "streams": batch.build_streams()},
            "mixed": {"value": q * args.steps / tmx, "unit": UNIT, "ms_per_step": 1e3 * tmx / args.steps,
                      "mixed_threshold": args.mixed_threshold,
                      "accuracy": {"max_abs_dJ": float((Jmx - J64).abs().max()),
@@ -526,7 +526,7 @@ def run_native(args):
     M = mol.n_sph
     ctx = E.Context(mol, device=local).plan(E.ScreeningOptions(integral_threshold=tau,
                                                                mixed_threshold=args.mixed_threshold))
-    if args.streams > 1:
+    if args.streams > 0:
         ctx.set_tuning(streams=args.streams)
     prof = ctx.profile()
     quartets = prof["quartets"]
@@ -677,7 +677,7 @@ def run_native(args):
         "config": {"workload": args.config, "description": wdesc, "M": M, "quartets_per_build": quartets,
                    "primitive_quartets_per_build": prof["primitive_quartets"],
                    "flops_per_build_model": prof["flops"], "parallelism": f"replicas{ws}",
-                   "streams": args.streams,
+                   "streams": ctx.build_streams(mixed=True),
                    "l2": "inputs larger than L2 (D, J, K are M*M*8 bytes each)" if flush is None else
                          "L2 flushed between timed builds (256 MB write)",
                    "mixed_threshold": "per class (mixed_autotune)" if tune else args.mixed_threshold,
@@ -724,8 +724,8 @@ def main():
     ap.add_argument("--config", default="cfg4")
     ap.add_argument("--mixed-threshold", type=float, default=1e-9)
     ap.add_argument("--no-cpu-baseline", action="store_true")
-    ap.add_argument("--streams", type=int, default=1,
-                    help="streams the class launches of a build spread over (1..4)")
+    ap.add_argument("--streams", type=int, default=0,
+                    help="streams the class launches of a build spread over (1..4; 0 = by the plan's size)")
     ap.add_argument("--no-extra", action="store_true",
                     help="skip the incremental, ERI-stream and one-electron legs")
     ap.add_argument("--no-autotune", action="store_true",

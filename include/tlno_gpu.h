@@ -324,11 +324,12 @@ void* tlno_gpu_batch_stream(tlno_gpu_batch* b);
  * the shared-memory budget; 1..8 = the warp-per-quartet kernel with that many
  * warps; (dd|dd), (dd|dp) and (fp|dp) keep the block kernel where they have it), persistent grid multiplier
  * (the compile-time kernels size their grid from the occupancy calculator,
- * capped by grid_mult x SMs), and streams (1..4): the class launches of a
+ * capped by grid_mult x SMs), and streams (0..4): the class launches of a
  * build spread over that many streams (parallel branches of a captured
  * graph), so that the tail of one class overlaps the next; 1 keeps them in
- * order on the context's stream.  Without this call a short build spreads
- * over up to 8 streams and a long one keeps them in order.  A per-class-combination generic override
+ * order on the context's stream; 0, also without this call, decides by the
+ * plan's size: a short build spreads over up to 8 streams, a long one keeps
+ * them in order.  A per-class-combination generic override
  * is set separately. */
 typedef struct {
     int generic_bk;
@@ -344,6 +345,10 @@ int tlno_gpu_batch_set_tuning(tlno_gpu_batch* b, const tlno_gpu_tuning* t);
  * while they fit, and a class combination of which one has none runs the
  * warp-per-quartet kernel. */
 int tlno_gpu_set_projector_limit(tlno_gpu_context* ctx, long long bytes);
+/* Streams a build of the current plan spreads its class launches over (flags:
+ * 0 or TLNO_GPU_MIXED). */
+int tlno_gpu_build_streams(const tlno_gpu_context* ctx, int flags);
+int tlno_gpu_batch_build_streams(const tlno_gpu_batch* b, int flags);
 int tlno_gpu_set_combo_generic(tlno_gpu_context* ctx, int combo_id, int force_generic);
 /* Per class-combination statistics of the current plan: for i < n, writes
  * (X, Y, la, lb, lc, ld, fast, n_tiles) into ints[8*i] and

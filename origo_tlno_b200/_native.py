@@ -133,6 +133,8 @@ def lib() -> C.CDLL:
         "tlno_gpu_batch_stream": (_vp, [_vp]),
         "tlno_gpu_set_tuning": (C.c_int, [_vp, C.POINTER(Tuning)]),
         "tlno_gpu_set_projector_limit": (C.c_int, [_vp, C.c_longlong]),
+        "tlno_gpu_build_streams": (C.c_int, [_vp, C.c_int]),
+        "tlno_gpu_batch_build_streams": (C.c_int, [_vp, C.c_int]),
         "tlno_gpu_set_combo_generic": (C.c_int, [_vp, C.c_int, C.c_int]),
         "tlno_gpu_plan_combos": (C.c_int, [_vp, C.c_int, _vp, _vp]),
         "tlno_gpu_time_combo": (C.c_int, [_vp, C.c_int, C.c_int, C.c_int, _dp]),
@@ -178,6 +180,6 @@ EXPORTED = [
     "tlno_gpu_batch_destroy", "tlno_gpu_batch_total_elements", "tlno_gpu_batch_offsets",
     "tlno_gpu_batch_profile", "tlno_gpu_batch_jk", "tlno_gpu_batch_graph_capture",
     "tlno_gpu_batch_graph_launch", "tlno_gpu_batch_synchronize", "tlno_gpu_batch_stream",
-    "tlno_gpu_set_tuning", "tlno_gpu_set_projector_limit", "tlno_gpu_set_combo_generic", "tlno_gpu_plan_combos", "tlno_gpu_time_combo",
+    "tlno_gpu_set_tuning", "tlno_gpu_build_streams", "tlno_gpu_batch_build_streams", "tlno_gpu_set_projector_limit", "tlno_gpu_set_combo_generic", "tlno_gpu_plan_combos", "tlno_gpu_time_combo",
     "tlno_gpu_set_class_tuning", "tlno_gpu_class_jk", "tlno_gpu_batch_set_tuning",
 ]

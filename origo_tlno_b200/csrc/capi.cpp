@@ -196,7 +196,27 @@ int fan_streams(const Plan2e& plan, const Tuning& tune, std::size_t launches) {
     if (plan.total_flops >= kFanMaxFlops) return 1;
     return static_cast<int>(std::min<std::size_t>(8, std::max<std::size_t>(launches, 1)));
 }
+
+// The launches of a build: per class one, or (mixed build) the FP64 and the
+// FP32 pass.  A class whose split multiplier is 0 stays FP64 in a mixed build
+// (one launch, no FP32 pass).
+struct ClassPass {
+    std::size_t ci;
+    int pass;
+};
+std::vector<ClassPass> class_passes(const Plan2e& plan, bool mixed) {
+    std::vector<ClassPass> out;
+    for (std::size_t ci = 0; ci < plan.combos.size(); ++ci) {
+        const bool split = mixed && plan.combos[ci].mix_scale > 0.0;
+        for (int pass = 0; pass < (split ? 2 : 1); ++pass) out.push_back({ci, pass});
+    }
+    return out;
+}
 }  // namespace
+
+int build_streams(const Plan2e& plan, const Tuning& tune, bool mixed) {
+    return fan_streams(plan, tune, class_passes(plan, mixed).size());
+}
 
 void enqueue_jk(Plan2e& plan, const Tuning& tune, const BuildSpec& spec, const double* dD, double* dJ,
                 double* dK, long long total, int M_single, double* d_dmax, float* dD32, cudaStream_t s,
@@ -225,18 +245,7 @@ void enqueue_jk(Plan2e& plan, const Tuning& tune, const BuildSpec& spec, const d
     int sms = 0, devid = 0;
     TLNO_CUDA(cudaGetDevice(&devid));
     TLNO_CUDA(cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, devid));
-    // The launches of the build: per class one, or (mixed build) the FP64 and
-    // the FP32 pass.  A class whose split multiplier is 0 stays FP64 in a mixed
-    // build (one launch, no FP32 pass).
-    struct Launch {
-        std::size_t ci;
-        int pass;
-    };
-    std::vector<Launch> launches;
-    for (std::size_t ci = 0; ci < plan.combos.size(); ++ci) {
-        const bool split = mixed && plan.combos[ci].mix_scale > 0.0;
-        for (int pass = 0; pass < (split ? 2 : 1); ++pass) launches.push_back({ci, pass});
-    }
+    std::vector<ClassPass> launches = class_passes(plan, mixed);
     // Launches over `nst` streams: fork after the shared prologue (zeroing,
     // max|D|, density tables), each launch on the stream with the least flops
     // so far (largest classes first), join before the symmetrisation.  J and K
@@ -245,7 +254,7 @@ void enqueue_jk(Plan2e& plan, const Tuning& tune, const BuildSpec& spec, const d
     StreamBranches branches(fan, s, nst);
     std::vector<int> stream_of(launches.size(), 0);
     if (nst > 1) {
-        std::stable_sort(launches.begin(), launches.end(), [&](const Launch& x, const Launch& y) {
+        std::stable_sort(launches.begin(), launches.end(), [&](const ClassPass& x, const ClassPass& y) {
             return plan.combos[x.ci].flops > plan.combos[y.ci].flops;
         });
         std::vector<double> load(nst, 0.0);
@@ -947,12 +956,16 @@ int tlno_gpu_synchronize(tlno_gpu_context* ctx) {
 
 void* tlno_gpu_stream(tlno_gpu_context* ctx) { return ctx ? static_cast<void*>(ctx->stream) : nullptr; }
 
+static void check_tuning(const tlno_gpu_tuning& t) {
+    if (t.generic_bk < 1 || t.generic_bk > 4096 || t.generic_warps < 0 || t.generic_warps > 8 || t.grid_mult < 1 ||
+        t.grid_mult > 64 || t.streams < 0 || t.streams > 4)
+        throw Error(TLNO_GPU_E_INVALID, "tlno_gpu: tuning value out of range");
+}
+
 int tlno_gpu_set_tuning(tlno_gpu_context* ctx, const tlno_gpu_tuning* t) {
     return guarded([&] {
         if (!ctx || !t) throw Error(TLNO_GPU_E_INVALID, "tlno_gpu: null argument");
-        if (t->generic_bk < 1 || t->generic_bk > 4096 || t->generic_warps < 0 || t->generic_warps > 8 ||
-            t->grid_mult < 1 || t->grid_mult > 64 || t->streams < 1 || t->streams > 4)
-            throw Error(TLNO_GPU_E_INVALID, "tlno_gpu: tuning value out of range");
+        check_tuning(*t);
         ctx->tune.streams = t->streams;
         ctx->tune.generic_bk = t->generic_bk;
         ctx->tune.generic_warps = t->generic_warps;
@@ -965,6 +978,24 @@ int tlno_gpu_set_projector_limit(tlno_gpu_context* ctx, long long bytes) {
         if (!ctx || bytes < 0) throw Error(TLNO_GPU_E_INVALID, "tlno_gpu: projector limit must be >= 0");
         ctx->tune.max_projector_bytes = bytes;
     });
+}
+
+int tlno_gpu_build_streams(const tlno_gpu_context* ctx, int flags) {
+    int n = 0;
+    const int rc = guarded([&] {
+        if (!ctx || !ctx->plan) throw Error(TLNO_GPU_E_STATE, "tlno_gpu: no plan; call tlno_gpu_plan first");
+        n = build_streams(*ctx->plan, ctx->tune, flags & TLNO_GPU_MIXED);
+    });
+    return rc == TLNO_GPU_OK ? n : rc;
+}
+
+int tlno_gpu_batch_build_streams(const tlno_gpu_batch* b, int flags) {
+    int n = 0;
+    const int rc = guarded([&] {
+        if (!b) throw Error(TLNO_GPU_E_INVALID, "tlno_gpu: null batch");
+        n = build_streams(b->plan, b->tune, flags & TLNO_GPU_MIXED);
+    });
+    return rc == TLNO_GPU_OK ? n : rc;
 }
 
 int tlno_gpu_set_combo_generic(tlno_gpu_context* ctx, int combo_id, int force_generic) {
@@ -1175,9 +1206,7 @@ void tlno_gpu_batch_destroy(tlno_gpu_batch* b) { delete b; }
 int tlno_gpu_batch_set_tuning(tlno_gpu_batch* b, const tlno_gpu_tuning* t) {
     return guarded([&] {
         if (!b || !t) throw Error(TLNO_GPU_E_INVALID, "tlno_gpu: null argument");
-        if (t->generic_bk < 1 || t->generic_bk > 4096 || t->generic_warps < 0 || t->generic_warps > 8 ||
-            t->grid_mult < 1 || t->grid_mult > 64 || t->streams < 1 || t->streams > 4)
-            throw Error(TLNO_GPU_E_INVALID, "tlno_gpu: tuning value out of range");
+        check_tuning(*t);
         b->tune.generic_warps = t->generic_warps;
         b->tune.grid_mult = t->grid_mult;
         b->tune.streams = t->streams;

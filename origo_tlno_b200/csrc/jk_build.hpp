@@ -51,6 +51,9 @@ void enqueue_jk(Plan2e& plan, const Tuning& tune, const BuildSpec& spec, const d
                 double* dK, long long total, int M_single, double* d_dmax, float* dD32, cudaStream_t s,
                 StreamFan* fan = nullptr);
 
+// Streams such a build spreads its class launches over.
+int build_streams(const Plan2e& plan, const Tuning& tune, bool mixed);
+
 // Two-electron plan of a context's basis for the shell-level screen of o.
 std::unique_ptr<Plan2e> make_plan(const tlno_gpu_context* ctx, const tlno_gpu_screening& o);
 

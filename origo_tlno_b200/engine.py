@@ -228,13 +228,18 @@ class Context:
         N.check(N.lib().tlno_gpu_set_onee_thresholds(self.h, decay_eps, nuclear_eps))
 
     # -- tuning ---------------------------------------------------------
-    def set_tuning(self, generic_bk=64, generic_warps=0, grid_mult=8, streams=1):
+    def set_tuning(self, generic_bk=64, generic_warps=0, grid_mult=8, streams=0):
+        """Kernel schedule; streams 0 = by the plan's size, 1 = launches in order."""
         t = N.Tuning(generic_bk, generic_warps, grid_mult, streams)
         N.check(N.lib().tlno_gpu_set_tuning(self.h, C.byref(t)))
 
     def set_projector_limit(self, nbytes: int):
         """Device memory the next plan may spend on pair-projector tables."""
         N.check(N.lib().tlno_gpu_set_projector_limit(self.h, nbytes))
+
+    def build_streams(self, mixed=False) -> int:
+        """Streams a build spreads its class launches over."""
+        return N.check(N.lib().tlno_gpu_build_streams(self.h, N.MIXED if mixed else 0))
 
     def set_combo_generic(self, combo_id: int, force: bool):
         N.check(N.lib().tlno_gpu_set_combo_generic(self.h, combo_id, 1 if force else 0))
@@ -291,9 +296,13 @@ class Batch:
         N.check(N.lib().tlno_gpu_batch_profile(self.h, C.byref(p)))
         return {f: getattr(p, f) for f, _ in N.Profile._fields_}
 
-    def set_tuning(self, generic_bk=64, generic_warps=0, grid_mult=8, streams=1):
+    def set_tuning(self, generic_bk=64, generic_warps=0, grid_mult=8, streams=0):
+        """Kernel schedule; streams 0 = by the plan's size, 1 = launches in order."""
         t = N.Tuning(generic_bk, generic_warps, grid_mult, streams)
         N.check(N.lib().tlno_gpu_batch_set_tuning(self.h, C.byref(t)))
+
+    def build_streams(self, mixed=False) -> int:
+        return N.check(N.lib().tlno_gpu_batch_build_streams(self.h, N.MIXED if mixed else 0))
 
     def jk(self, densities, mixed=False):
         D = np.concatenate([_f64(d).ravel() for d in densities])

@@ -45,3 +45,30 @@ def test_failed_build_leaves_nothing_running_beside_its_stream():
     ctx.synchronize()
     assert max(_maxabs(J.cpu().numpy(), ref["J"]), _maxabs(K.cpu().numpy(), ref["K"])) < 1e-12
     ctx.close()
+
+
+def test_tuning_another_knob_keeps_the_streams_of_the_plans_size():
+    # streams 0 (the default) means by the plan's size: it can be set back, and
+    # setting another knob does not put a short build on one stream
+    ctx = E.Context(M.cfg1()).plan(E.ScreeningOptions(integral_threshold=1e-12))
+    auto = ctx.build_streams()
+    assert auto == 8 and ctx.build_streams(mixed=True) == 8
+    ctx.set_tuning(grid_mult=8)
+    assert ctx.build_streams() == auto
+    for n in (1, 4):
+        ctx.set_tuning(streams=n)
+        assert ctx.build_streams() == n
+    ctx.set_tuning(streams=0)
+    assert ctx.build_streams() == auto
+    b = E.Batch([ctx], E.ScreeningOptions(integral_threshold=1e-12))
+    b.set_tuning(streams=2)
+    assert b.build_streams() == 2
+    b.set_tuning()
+    assert b.build_streams() == auto
+    for bad in (-1, 5):
+        with pytest.raises(E.TlnoError, match="out of range"):
+            ctx.set_tuning(streams=bad)
+        with pytest.raises(E.TlnoError, match="out of range"):
+            b.set_tuning(streams=bad)
+    b.close()
+    ctx.close()
