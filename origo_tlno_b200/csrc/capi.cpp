@@ -219,9 +219,10 @@ int build_streams(const Plan2e& plan, const Tuning& tune, bool mixed) {
 }
 
 void enqueue_jk(Plan2e& plan, const Tuning& tune, const BuildSpec& spec, const double* dD, double* dJ,
-                double* dK, long long total, int M_single, double* d_dmax, float* dD32, cudaStream_t s,
+                double* dK, long long total, double* d_dmax, float* dD32, cudaStream_t s,
                 StreamFan* fan) {
     const bool want_j = spec.want_j, want_k = spec.want_k, mixed = spec.mixed;
+    const int M_single = plan.n_mol == 1 ? plan.mol_M[0] : 0;
     launch_clear_build(dJ, dK, total, plan.d_counters.as<int>(), static_cast<int>(2 * plan.combos.size()), s);
     if (mixed) launch_absmax_f32(dD, total, d_dmax, dD32, s);
     dev::DensityScreen den{};
@@ -456,7 +457,7 @@ void run_jk(tlno_gpu_context* ctx, const double* density, double* J, double* K, 
         const bool pk = den ? out_k : (out_k || want_g);
         BuildSpec spec = spec_from(eo, pj, pk, mixed, false);
         spec.fail_after = std::exchange(ctx->fail_after, -1);
-        enqueue_jk(*ctx->plan, ctx->tune, spec, dD, dJ, dK, n, M,
+        enqueue_jk(*ctx->plan, ctx->tune, spec, dD, dJ, dK, n,
                    ctx->w.dmax.as<double>(), d32, s, &thread_fan(ctx->device));
         if (!dev_ptrs) {
             if (out_j) TLNO_CUDA(cudaMemcpyAsync(J, dJ, sizeof(double) * n, cudaMemcpyDeviceToHost, s));
@@ -469,7 +470,7 @@ void run_jk(tlno_gpu_context* ctx, const double* density, double* J, double* K, 
         if (den) {
             gJ = ctx->w.J.as<double>();
             gK = ctx->w.K.as<double>();
-            enqueue_jk(*ctx->plan, ctx->tune, spec_from(eo, true, true, mixed, true), dD, gJ, gK, n, M,
+            enqueue_jk(*ctx->plan, ctx->tune, spec_from(eo, true, true, mixed, true), dD, gJ, gK, n,
                        ctx->w.dmax.as<double>(), d32, s, &thread_fan(ctx->device));
         }
         double* dG = G;
@@ -925,7 +926,7 @@ int tlno_gpu_jk_graph_capture(tlno_gpu_context* ctx, const double* d_density, do
         spec.fail_after = std::exchange(ctx->fail_after, -1);
         TLNO_CUDA(cudaStreamBeginCapture(ctx->stream, cudaStreamCaptureModeThreadLocal));
         try {
-            enqueue_jk(*ctx->plan, ctx->tune, spec, d_density, d_J, d_K, n, M, ctx->w.dmax.as<double>(), d32,
+            enqueue_jk(*ctx->plan, ctx->tune, spec, d_density, d_J, d_K, n, ctx->w.dmax.as<double>(), d32,
                        ctx->stream, &thread_fan(ctx->device));
         } catch (...) {
             cudaGraph_t g = nullptr;
@@ -1262,7 +1263,7 @@ int tlno_gpu_batch_jk(tlno_gpu_batch* b, const double* density, double* J, doubl
         validate_build_combination(b->screening);
         if (b->screening.density_threshold > 0.0) ensure_density_tables(b->plan);
         enqueue_jk(b->plan, b->tune, spec_from(b->screening, true, true, flags & TLNO_GPU_MIXED, false), dD, dJ, dK,
-                   b->total, 0, b->w.dmax.as<double>(), d32, s, &thread_fan(b->device));
+                   b->total, b->w.dmax.as<double>(), d32, s, &thread_fan(b->device));
         if (!dev_ptrs) {
             TLNO_CUDA(cudaMemcpyAsync(J, dJ, sizeof(double) * b->total, cudaMemcpyDeviceToHost, s));
             TLNO_CUDA(cudaMemcpyAsync(K, dK, sizeof(double) * b->total, cudaMemcpyDeviceToHost, s));
@@ -1288,7 +1289,7 @@ int tlno_gpu_batch_graph_capture(tlno_gpu_batch* b, const double* d_density, dou
         const BuildSpec spec = spec_from(b->screening, true, true, flags & TLNO_GPU_MIXED, false);
         TLNO_CUDA(cudaStreamBeginCapture(b->stream, cudaStreamCaptureModeThreadLocal));
         try {
-            enqueue_jk(b->plan, b->tune, spec, d_density, d_J, d_K, b->total, 0, b->w.dmax.as<double>(), d32,
+            enqueue_jk(b->plan, b->tune, spec, d_density, d_J, d_K, b->total, b->w.dmax.as<double>(), d32,
                        b->stream, &thread_fan(b->device));
         } catch (...) {
             cudaGraph_t g = nullptr;

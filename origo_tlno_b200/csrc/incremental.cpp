@@ -147,7 +147,7 @@ int update(tlno_gpu_incremental* st, const double* density, bool force, int flag
         d32 = st->D32.as<float>();
     }
     enqueue_jk(*st->plan, ctx->tune, spec_from(bo, true, true, mixed, true), in, st->J.as<double>(),
-               st->K.as<double>(), n, st->M, st->dmax.as<double>(), d32, s, &thread_fan(ctx->device));
+               st->K.as<double>(), n, st->dmax.as<double>(), d32, s, &thread_fan(ctx->device));
     launch_combine_g(st->J.as<double>(), st->K.as<double>(), st->Gb.as<double>(), n, s);
     // 4. next G with the reference's non-finite checks
     launch_g_accumulate(exact ? nullptr : st->G.as<double>(), st->Gb.as<double>(), st->Gnext.as<double>(), n,

@@ -53,3 +53,26 @@ def test_projector_limit_and_warp_form_give_the_same_matrices():
     with pytest.raises(E.TlnoError, match="limit"):
         ctx.set_projector_limit(-1)
     ctx.close()
+
+
+def test_batch_of_one_molecule_matches_its_context():
+    import torch
+    mol = M.water_cluster(2, seed=5, grid=(2, 1, 1))
+    D = M.random_density(mol.n_sph, max(1, mol.n_sph // 5), seed=6)
+    for opts in (E.ScreeningOptions(integral_threshold=1e-12, mixed_threshold=1e-6),
+                 E.ScreeningOptions(integral_threshold=1e-12, density_threshold=1e-9)):
+        ctx = E.Context(mol).plan(opts)
+        b = E.Batch([ctx], opts)
+        for mixed in (False, True):
+            ref = ctx.jk(D, mixed=mixed)
+            J, K = b.jk([D], mixed=mixed)
+            assert max(np.max(np.abs(J[0] - ref["J"])), np.max(np.abs(K[0] - ref["K"]))) < 1e-12
+            d = torch.tensor(D, device="cuda")
+            dJ, dK = torch.empty_like(d), torch.empty_like(d)
+            torch.cuda.synchronize()
+            b.graph_capture(d.data_ptr(), dJ.data_ptr(), dK.data_ptr(), mixed=mixed)
+            b.graph_launch()
+            b.synchronize()
+            assert max(np.max(np.abs(dJ.cpu().numpy() - ref["J"])), np.max(np.abs(dK.cpu().numpy() - ref["K"]))) < 1e-12
+        b.close()
+        ctx.close()
