@@ -815,8 +815,10 @@ void build_plan(Plan2e& plan, const std::vector<const Basis*>& bases, std::vecto
                         bd.lb = ts.lb;
                         cs.blocks.push_back(bd);
                         cs.prefix.push_back(cs.prefix.back() + nt);
+                        // (a pair of 220-primitive shells passes 31 bits)
+                        const long long tile_steps = (1LL * npb * npk * (w1 - w0)) >> (ts.lk + ts.lb);
                         int lg = 0;
-                        while ((npb * npk * (w1 - w0) >> (ts.lk + ts.lb)) >> (lg + 1)) ++lg;
+                        while (lg < 31 && tile_steps >> (lg + 1)) ++lg;
                         cost.push_back(lg);
                     }
                 }

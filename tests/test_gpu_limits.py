@@ -76,3 +76,14 @@ def test_batch_of_one_molecule_matches_its_context():
             assert max(np.max(np.abs(dJ.cpu().numpy() - ref["J"])), np.max(np.abs(dK.cpu().numpy() - ref["K"]))) < 1e-12
         b.close()
         ctx.close()
+
+
+def test_plan_of_a_contraction_beyond_31_bits():
+    # one shell of 220 primitives: 48400 primitive pairs, 2.3e9 primitive
+    # quartets in its one tile (planned with the decay metric, which evaluates
+    # no integral; the build itself is not run)
+    mol = M.Molecule("deep", np.array([1]), np.zeros((1, 3)))
+    mol.shells = [M.ShellSpec((0.0, 0.0, 0.0), 0, np.geomspace(0.1, 1e4, 220), np.ones(220), 0)]
+    ctx = E.Context(mol).plan(E.ScreeningOptions(integral_threshold=0.0, decay_threshold=1e-10))
+    assert ctx.profile()["primitive_quartets"] == 48400 ** 2
+    ctx.close()
