@@ -564,7 +564,7 @@ template <typename R, int LA, int LB, int LC, int LD>
 __global__ void __launch_bounds__(32 * FastShape<LA, LB, LC, LD>::WARPS, fast_min_blocks<R, LA, LB, LC, LD>())
     eri_fast_jk_kernel(PlanView pv, ClassLaunch cl) {
     using S = FastShape<LA, LB, LC, LD>;
-    extern __shared__ double fast_smem[];
+    extern __shared__ __align__(16) double fast_smem[];  // 16-byte records and vectors
     const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
     const int grp = warp / S::TPQ, g = warp % S::TPQ;
     // A quartet owned by one thread keeps its (a0|cd) rows in registers; a

@@ -303,7 +303,7 @@ __host__ __device__ constexpr int rows_min_blocks(int ch) { return ch == 1 ? 5 :
 template <typename R, int LC, int LD>
 __global__ void __launch_bounds__(rows_max_threads(RowsKet<LC, LD>::CH), rows_min_blocks(RowsKet<LC, LD>::CH))
     eri_rows_jk_kernel(PlanView pv, ClassLaunch cl, int nb_items, int part) {
-    extern __shared__ double smem[];
+    extern __shared__ __align__(16) double smem[];  // the G rows are read as 16-byte vectors
     RowsLayout lay;
     lay.init(cl.la, cl.lb, LC, LD, nb_items);
     __shared__ int s_tile;
