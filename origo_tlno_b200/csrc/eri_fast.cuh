@@ -487,19 +487,6 @@ __host__ __device__ constexpr int fast_min_blocks() {
     return 4;
 }
 
-// Where a bra-group class keeps the per-tile density values of a lane:
-// 0 none (no bra groups), 1 registers, 2 shared memory.  Shared memory where
-// registers are tight (FP64, and the capped FP32 classes: 3-10% faster on the
-// s/p classes of 400 waters); registers for the uncapped FP32 classes, where
-// the extra shared memory costs resident CTAs (+18% on (pp|ps)).
-template <typename R, int LA, int LB, int LC, int LD>
-__host__ __device__ constexpr int fast_pre_mode() {
-    using S = FastShape<LA, LB, LC, LD>;
-    if (S::PRE_VALS == 0) return 0;
-    if (std::is_same<R, double>::value) return 2;
-    return fast_min_blocks<R, LA, LB, LC, LD>() > 1 ? 2 : 1;
-}
-
 // Whether the sums carried across a block's bras live in shared memory: FP64
 // (ps|ps), whose 15 sums then leave room for 4 resident CTAs without spills
 // (91 waters 35.4 -> 33.6 ms, without digestion 25.2 -> 21.3 ms).  (ss|ss),
@@ -553,10 +540,9 @@ __host__ __device__ constexpr int fast_region_bytes() {
     using S = FastShape<LA, LB, LC, LD>;
     const int jab = fast_jab_smem<R, LA, LB, LC, LD>() ? S::TPQ * S::NSAB * 33 : 0;
     if (!fast_async<R, LA, LB, LC, LD>()) return (jab * static_cast<int>(sizeof(R)) + 15) / 16 * 16;
-    const int pre = fast_pre_mode<R, LA, LB, LC, LD>() == 2 ? S::PRE_VALS : 0;
     const int car = fast_carry_smem<R, LA, LB, LC, LD>() ? S::PRE_VALS : 0;
     const int bytes = (S::GB > 1 ? S::GB * (static_cast<int>(sizeof(PairRec)) + 4) : 0) +
-                      (S::GB * S::NSAB + 32 * (S::OWN_VALS + pre + car) + jab) * static_cast<int>(sizeof(R));
+                      (S::GB * S::NSAB + 32 * (S::OWN_VALS + S::PRE_VALS + car) + jab) * static_cast<int>(sizeof(R));
     return (bytes + 15) / 16 * 16;
 }
 
@@ -593,7 +579,6 @@ __global__ void __launch_bounds__(32 * FastShape<LA, LB, LC, LD>::WARPS, fast_mi
     // The warp group's region: (bra-group classes) the pair records of the
     // block's bras; D[a,b] of the bras; the asynchronous density values of a
     // quartet; (bra-group classes) the per-tile density values.
-    constexpr int PRE_MODE = fast_pre_mode<R, LA, LB, LC, LD>();
     constexpr bool GROUP = S::GB > 1;
     constexpr bool ASYNC = fast_async<R, LA, LB, LC, LD>();
     unsigned char* wsm = reinterpret_cast<unsigned char*>(fast_smem) + smem_used +
@@ -603,7 +588,7 @@ __global__ void __launch_bounds__(32 * FastShape<LA, LB, LC, LD>::WARPS, fast_mi
     R* wdab = reinterpret_cast<R*>(wsm + (GROUP ? S::GB * (sizeof(PairRec) + sizeof(int)) : 0));
     R* dg = wdab + S::GB * S::NSAB;
     R* pre = dg + S::OWN_VALS * 32;
-    R* carry = pre + (PRE_MODE == 2 ? S::PRE_VALS * 32 : 0);
+    R* carry = pre + S::PRE_VALS * 32;
     R* jred = ASYNC ? carry + (fast_carry_smem<R, LA, LB, LC, LD>() ? S::PRE_VALS * 32 : 0)
                     : reinterpret_cast<R*>(wsm);
     int staged = -1;               // block whose bras are staged
@@ -740,14 +725,11 @@ __global__ void __launch_bounds__(32 * FastShape<LA, LB, LC, LD>::WARPS, fast_mi
         }
         // The bras of a block share shell A, so the lane's D[a, c], D[a, d]
         // and D[c, d] are the same for every bra of it: they are gathered once
-        // per tile, into registers or this lane's shared-memory slots
-        // [k * 32 + lane].
-        R preg[PRE_MODE == 1 ? S::PRE_VALS : 1];
-        auto pre_at = [&](int k) -> R& {
-            if constexpr (PRE_MODE == 1) return preg[k];
-            else return pre[k * 32 + lane];
-        };
-        if constexpr (PRE_MODE != 0) {
+        // per tile into this lane's shared-memory slots [k * 32 + lane]
+        // (registers are tight: 3-10% faster than keeping them there on the s/p
+        // classes of 400 waters).
+        auto pre_at = [&](int k) -> R& { return pre[k * 32 + lane]; };
+        if constexpr (GROUP) {
             const int a0b = wrec[0].a0;
             if (cl.want_k) {
 #pragma unroll
@@ -843,12 +825,12 @@ __global__ void __launch_bounds__(32 * FastShape<LA, LB, LC, LD>::WARPS, fast_mi
                 async_commit();
             }
             auto d_ac = [&](int sa, int sc) -> R {
-                if constexpr (PRE_MODE != 0) return pre_at(sa * S::NSC + sc);
+                if constexpr (GROUP) return pre_at(sa * S::NSC + sc);
                 else if constexpr (ASYNC) return dg[(sa * S::NSC + sc) * 32 + lane];
                 else return dm(a0 + sa, c0, sc);
             };
             auto d_ad = [&](int sa, int sd) -> R {
-                if constexpr (PRE_MODE != 0) return pre_at(S::NSA * S::NSC + sa * S::NSD + sd);
+                if constexpr (GROUP) return pre_at(S::NSA * S::NSC + sa * S::NSD + sd);
                 else if constexpr (ASYNC) return dg[(S::NSA * S::NSC + sa * S::NSD + sd) * 32 + lane];
                 else return dm(a0 + sa, d0, sd);
             };
@@ -862,7 +844,7 @@ __global__ void __launch_bounds__(32 * FastShape<LA, LB, LC, LD>::WARPS, fast_mi
             };
             auto d_cd = [&](int sc, int sd) -> R {
                 const int t = sc * S::NSD + sd;
-                if constexpr (PRE_MODE != 0) return pre_at(S::NSA * (S::NSC + S::NSD) + t);
+                if constexpr (GROUP) return pre_at(S::NSA * (S::NSC + S::NSD) + t);
                 else if constexpr (ASYNC) return dg[(CX + t) * 32 + lane];
                 else return dm(c0 + sc, d0, sd);
             };
