@@ -355,28 +355,37 @@ __device__ void generic_quartet(const PlanView& pv, const ClassLaunch& cl,
     __syncwarp();
 }
 
+// A warp's region: in shared memory, or (GLOBAL) in global scratch where one
+// region is larger than a block's shared memory ((gg|gg): 506 KB).
+template <bool GLOBAL>
+__device__ __forceinline__ double* warp_region(double* smem, double* scratch, int words) {
+    const int warp = threadIdx.x >> 5;
+    if constexpr (GLOBAL) return scratch + (static_cast<size_t>(blockIdx.x) * (blockDim.x >> 5) + warp) * words;
+    else return smem + warp * words;
+}
+
 // Explicit quartet list (STORE and SCHWARZ modes).
-template <typename R, int MODE>
-__global__ void eri_generic_list_kernel(PlanView pv, ClassLaunch cl) {
+template <typename R, int MODE, bool GLOBAL>
+__global__ void eri_generic_list_kernel(PlanView pv, ClassLaunch cl, double* scratch) {
     extern __shared__ double smem[];
     GenericLayout lay;
     lay.init(cl.la, cl.lb, cl.lc, cl.ld);
     const int warps = blockDim.x >> 5;
     const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
-    double* wsm = smem + warp * lay.words;
+    double* wsm = warp_region<GLOBAL>(smem, scratch, lay.words);
     for (int q = blockIdx.x * warps + warp; q < cl.n_quartets; q += gridDim.x * warps)
         generic_quartet<R, MODE>(pv, cl, lay, wsm, lane, cl.q_bra[q], cl.q_ket[q], q);
 }
 
 // Tiled schedule (J/K mode): tile = 1 bra pair x bk ket pairs.
-template <typename R>
-__global__ void eri_generic_jk_kernel(PlanView pv, ClassLaunch cl) {
+template <typename R, bool GLOBAL>
+__global__ void eri_generic_jk_kernel(PlanView pv, ClassLaunch cl, double* scratch) {
     extern __shared__ double smem[];
     GenericLayout lay;
     lay.init(cl.la, cl.lb, cl.lc, cl.ld);
     const int warps = blockDim.x >> 5;
     const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
-    double* wsm = smem + warp * lay.words;
+    double* wsm = warp_region<GLOBAL>(smem, scratch, lay.words);
     const double thr = (cl.prec_mode != 0) ? cl.tau_mix / fmax(*cl.dmax, 1e-300) : 0.0;
     int pb_bra = -1;  // bra pair whose projector this warp holds
     for (int tile = cl.tile_begin + blockIdx.x; tile < cl.tile_end; tile += gridDim.x) {
@@ -419,12 +428,15 @@ __global__ void eri_generic_jk_kernel(PlanView pv, ClassLaunch cl) {
 // pair_projector_kernel).
 //
 // Shared memory (doubles): region0 = max(NB item slots x 3 2-D tables,
-// X + V + the six density blocks), then the radial block T.
+// X + V + the six density blocks), then the radial block T.  X holds xc ket
+// columns at a time: all of them, or as many as fit beside T and V ((gg|gg):
+// T 164 KB, V 51 KB, 5 of 81 columns of X).
 struct GenericCtaLayout {
     int las, lcs, ks, gs, gslot, nas, ncs, na, nb, nc, nd, nsab, nscd;
     int nb_items;  // item slots per batch
+    int xc;        // ket columns of X per pass
     int off_X, off_V, off_P, off_T, words;
-    __host__ __device__ void init(int la, int lb, int lc, int ld, int nbi) {
+    __host__ __device__ void init(int la, int lb, int lc, int ld, int nbi, int xcols) {
         las = la + lb;
         lcs = lc + ld;
         ks = lcs + 1;
@@ -435,11 +447,12 @@ struct GenericCtaLayout {
         nsab = na * nb;
         nscd = nc * nd;
         nb_items = nbi;
+        xc = xcols;
         // odd slot size: the threads' own slots fall in different banks
         gslot = (3 * gs) | 1;
         const int g_words = nb_items * gslot;
         off_X = 0;
-        off_V = off_X + nas * nscd;
+        off_V = off_X + nas * xc;
         off_P = off_V + nsab * nscd;
         const int tail = off_P + na * nb + nc * nd + nb * nd + nb * nc + na * nd + na * nc;
         off_T = ((g_words > tail ? g_words : tail) + 1) & ~1;
@@ -553,21 +566,24 @@ __device__ void generic_quartet_cta(const PlanView& pv, const ClassLaunch& cl, c
     const double* PKt = pv.proj + pv.proj_off[ket];
     double* X = sm + lay.off_X;
     double* V = sm + lay.off_V;
-    for (int e = tid; e < lay.nas * lay.nscd; e += nt) {
-        const int ia = e / lay.nscd, s = e - ia * lay.nscd;
-        const R* trow = T + ia * lay.ncs;
-        double acc = 0.0;
-        for (int ic = 0; ic < lay.ncs; ++ic) acc += double(trow[ic]) * __ldg(PKt + ic * lay.nscd + s);
-        X[e] = acc;
+    for (int s0 = 0; s0 < lay.nscd; s0 += lay.xc) {
+        const int nx = min(lay.xc, lay.nscd - s0);
+        for (int e = tid; e < lay.nas * nx; e += nt) {
+            const int ia = e / nx, s = e - ia * nx;
+            const R* trow = T + ia * lay.ncs;
+            double acc = 0.0;
+            for (int ic = 0; ic < lay.ncs; ++ic) acc += double(trow[ic]) * __ldg(PKt + ic * lay.nscd + s0 + s);
+            X[ia * lay.xc + s] = acc;
+        }
+        __syncthreads();
+        for (int e = tid; e < lay.nsab * nx; e += nt) {
+            const int sab = e / nx, s = e - sab * nx;
+            double acc = 0.0;
+            for (int ia = 0; ia < lay.nas; ++ia) acc += __ldg(PBt + ia * lay.nsab + sab) * X[ia * lay.xc + s];
+            V[sab * lay.nscd + s0 + s] = acc;
+        }
+        __syncthreads();
     }
-    __syncthreads();
-    for (int e = tid; e < lay.nsab * lay.nscd; e += nt) {
-        const int sab = e / lay.nscd, s = e - sab * lay.nscd;
-        double acc = 0.0;
-        for (int ia = 0; ia < lay.nas; ++ia) acc += __ldg(PBt + ia * lay.nsab + sab) * X[ia * lay.nscd + s];
-        V[e] = acc;
-    }
-    __syncthreads();
 
     block_digest(pv, cl, lay, sm, V, br, kr, bra, ket, jon, kon);
 }
@@ -578,10 +594,10 @@ __device__ void generic_quartet_cta(const PlanView& pv, const ClassLaunch& cl, c
 // this kernel ran them, (ff|ff) of 14 f-shell atoms, 31 tiles of 393 quartets:
 // 1.66 -> 0.27 ms).
 template <typename R>
-__global__ void eri_generic_cta_jk_kernel(PlanView pv, ClassLaunch cl, int nb_items, int part) {
+__global__ void eri_generic_cta_jk_kernel(PlanView pv, ClassLaunch cl, int nb_items, int xc, int part) {
     extern __shared__ double smem[];
     GenericCtaLayout lay;
-    lay.init(cl.la, cl.lb, cl.lc, cl.ld, nb_items);
+    lay.init(cl.la, cl.lb, cl.lc, cl.ld, nb_items, xc);
     __shared__ int s_tile;
     const double thr = (cl.prec_mode != 0) ? cl.tau_mix / fmax(*cl.dmax, 1e-300) : 0.0;
     const int parts = (cl.bk + part - 1) / part;

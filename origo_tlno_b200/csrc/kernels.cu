@@ -500,11 +500,11 @@ void ensure_device_tables() {
     rows_upload(t, ct, c2s);
     TLNO_CUDA(cudaGetLastError());
     // The generic kernel may need more than 48 KB of dynamic shared memory.
-    const int maxsm = 227 * 1024;
-    TLNO_CUDA(cudaFuncSetAttribute(eri_generic_list_kernel<double, kStore>, cudaFuncAttributeMaxDynamicSharedMemorySize, maxsm));
-    TLNO_CUDA(cudaFuncSetAttribute(eri_generic_list_kernel<double, kSchwarz>, cudaFuncAttributeMaxDynamicSharedMemorySize, maxsm));
-    TLNO_CUDA(cudaFuncSetAttribute(eri_generic_jk_kernel<double>, cudaFuncAttributeMaxDynamicSharedMemorySize, maxsm));
-    TLNO_CUDA(cudaFuncSetAttribute(eri_generic_jk_kernel<float>, cudaFuncAttributeMaxDynamicSharedMemorySize, maxsm));
+    const int maxsm = kMaxWarpSmem;
+    TLNO_CUDA(cudaFuncSetAttribute(eri_generic_list_kernel<double, kStore, false>, cudaFuncAttributeMaxDynamicSharedMemorySize, maxsm));
+    TLNO_CUDA(cudaFuncSetAttribute(eri_generic_list_kernel<double, kSchwarz, false>, cudaFuncAttributeMaxDynamicSharedMemorySize, maxsm));
+    TLNO_CUDA(cudaFuncSetAttribute(eri_generic_jk_kernel<double, false>, cudaFuncAttributeMaxDynamicSharedMemorySize, maxsm));
+    TLNO_CUDA(cudaFuncSetAttribute(eri_generic_jk_kernel<float, false>, cudaFuncAttributeMaxDynamicSharedMemorySize, maxsm));
     // (the block-per-quartet kernel also holds a little static shared memory)
     TLNO_CUDA(cudaFuncSetAttribute(eri_generic_cta_jk_kernel<double>, cudaFuncAttributeMaxDynamicSharedMemorySize, maxsm - 1024));
     TLNO_CUDA(cudaFuncSetAttribute(eri_generic_cta_jk_kernel<float>, cudaFuncAttributeMaxDynamicSharedMemorySize, maxsm - 1024));
@@ -524,22 +524,44 @@ static int generic_warps_for(int bytes) {
     return w;
 }
 
-void launch_eri_store(const PlanView& pv, const ClassLaunch& cl, cudaStream_t s) {
+bool generic_needs_scratch(int la, int lb, int lc, int ld) {
+    return generic_warp_bytes(la, lb, lc, ld) > kMaxWarpSmem;
+}
+
+// Runs launch(grid, scratch) with the warp regions of a class of the
+// warp-per-quartet kernels in global memory: one warp per block and at most
+// 2 blocks per SM (150 MB for (gg|gg)), for the few quartets of such classes.
+template <class F>
+static void with_scratch(int bytes, long long units, cudaStream_t s, F&& launch) {
+    const int grid = static_cast<int>(std::min<long long>(units, sm_count() * 2));
+    void* scratch = nullptr;
+    TLNO_CUDA(cudaMallocAsync(&scratch, static_cast<std::size_t>(bytes) * grid, s));
+    launch(grid, static_cast<double*>(scratch));
+    const cudaError_t e = cudaGetLastError();
+    TLNO_CUDA(cudaFreeAsync(scratch, s));
+    TLNO_CUDA(e);
+}
+
+template <int MODE>
+static void launch_generic_list(const PlanView& pv, const ClassLaunch& cl, cudaStream_t s) {
     if (cl.n_quartets == 0) return;
     const int bytes = generic_warp_bytes(cl.la, cl.lb, cl.lc, cl.ld);
+    if (bytes > kMaxWarpSmem) {
+        with_scratch(bytes, cl.n_quartets, s, [&](int grid, double* scratch) {
+            eri_generic_list_kernel<double, MODE, true><<<grid, 32, 0, s>>>(pv, cl, scratch);
+        });
+        return;
+    }
     const int warps = generic_warps_for(bytes);
     const int grid = std::min((cl.n_quartets + warps - 1) / warps, sm_count() * 8);
-    eri_generic_list_kernel<double, kStore><<<grid, 32 * warps, bytes * warps, s>>>(pv, cl);
+    eri_generic_list_kernel<double, MODE, false><<<grid, 32 * warps, bytes * warps, s>>>(pv, cl, nullptr);
     TLNO_CUDA(cudaGetLastError());
 }
 
+void launch_eri_store(const PlanView& pv, const ClassLaunch& cl, cudaStream_t s) { launch_generic_list<kStore>(pv, cl, s); }
+
 void launch_eri_schwarz(const PlanView& pv, const ClassLaunch& cl, cudaStream_t s) {
-    if (cl.n_quartets == 0) return;
-    const int bytes = generic_warp_bytes(cl.la, cl.lb, cl.lc, cl.ld);
-    const int warps = generic_warps_for(bytes);
-    const int grid = std::min((cl.n_quartets + warps - 1) / warps, sm_count() * 8);
-    eri_generic_list_kernel<double, kSchwarz><<<grid, 32 * warps, bytes * warps, s>>>(pv, cl);
-    TLNO_CUDA(cudaGetLastError());
+    launch_generic_list<kSchwarz>(pv, cl, s);
 }
 
 void launch_pair_projectors(const int* pair_A, const int* pair_B, const double* shell_xyz, const int* shell_L,
@@ -558,18 +580,20 @@ void launch_pair_records(const PlanView& pv, int n_pairs, PairRec* out, cudaStre
     TLNO_CUDA(cudaGetLastError());
 }
 
-// CTA shape of the generic J/K kernel for a class: threads per block and item
-// slots per batch, and the dynamic shared memory it needs.
-static void generic_cta_shape(int la, int lb, int lc, int ld, int& threads, int& nb_items, int& bytes) {
+// CTA shape of the generic J/K kernel for a class: threads per block, item
+// slots per batch, ket columns of X per pass and the dynamic shared memory.
+static void generic_cta_shape(int la, int lb, int lc, int ld, int& threads, int& nb_items, int& xc, int& bytes) {
     GenericCtaLayout lay;
-    lay.init(la, lb, lc, ld, 1);
+    xc = nsph(lc) * nsph(ld);
+    lay.init(la, lb, lc, ld, 1, xc);
     threads = lay.nas * lay.ncs > 2048 ? 256 : 128;
     nb_items = 64;
     for (;;) {
-        lay.init(la, lb, lc, ld, nb_items);
+        lay.init(la, lb, lc, ld, nb_items, xc);
         if (lay.words * 8 <= 100 * 1024 || nb_items <= 16) break;
         nb_items /= 2;
     }
+    while (lay.words * 8 > kMaxBlockSmem && xc > 1) lay.init(la, lb, lc, ld, nb_items, --xc);
     bytes = lay.words * 8;
 }
 
@@ -580,8 +604,8 @@ void launch_eri_jk_generic(const PlanView& pv, const ClassLaunch& cl, bool fp32,
         if (!pv.proj) throw Error(-3, "tlno_gpu: block-per-quartet launch without projectors");
         if (launch_eri_jk_rows(pv, cl, fp32, sm_count(), s)) return;
         // one quartet per block at a time, projectors from the plan
-        int threads = 0, nb_items = 0, bytes = 0;
-        generic_cta_shape(cl.la, cl.lb, cl.lc, cl.ld, threads, nb_items, bytes);
+        int threads = 0, nb_items = 0, xc = 0, bytes = 0;
+        generic_cta_shape(cl.la, cl.lb, cl.lc, cl.ld, threads, nb_items, xc, bytes);
         int per_sm = 0;
         if (fp32) {
             TLNO_CUDA(cudaOccupancyMaxActiveBlocksPerMultiprocessor(&per_sm, eri_generic_cta_jk_kernel<float>, threads, bytes));
@@ -593,22 +617,29 @@ void launch_eri_jk_generic(const PlanView& pv, const ClassLaunch& cl, bool fp32,
         const int part = block_tile_part(ntiles, cl.bk, wave);
         const int g = static_cast<int>(std::max(1LL, std::min<long long>(ntiles * ((cl.bk + part - 1) / part), wave)));
         if (fp32)
-            eri_generic_cta_jk_kernel<float><<<g, threads, bytes, s>>>(pv, cl, nb_items, part);
+            eri_generic_cta_jk_kernel<float><<<g, threads, bytes, s>>>(pv, cl, nb_items, xc, part);
         else
-            eri_generic_cta_jk_kernel<double><<<g, threads, bytes, s>>>(pv, cl, nb_items, part);
+            eri_generic_cta_jk_kernel<double><<<g, threads, bytes, s>>>(pv, cl, nb_items, xc, part);
         TLNO_CUDA(cudaGetLastError());
         return;
     }
     const int bytes = generic_warp_bytes(cl.la, cl.lb, cl.lc, cl.ld);
+    if (bytes > kMaxWarpSmem) {
+        with_scratch(bytes, cl.tile_end - cl.tile_begin, s, [&](int g, double* scratch) {
+            if (fp32) eri_generic_jk_kernel<float, true><<<g, 32, 0, s>>>(pv, cl, scratch);
+            else eri_generic_jk_kernel<double, true><<<g, 32, 0, s>>>(pv, cl, scratch);
+        });
+        return;
+    }
     if (warps <= 0) warps = generic_warps_for(bytes);
     while (warps > 1 && bytes * warps > 200 * 1024) --warps;
     const int ntiles = cl.tile_end - cl.tile_begin;
     if (grid <= 0) grid = sm_count() * 4;
     grid = std::min(grid, ntiles);
     if (fp32)
-        eri_generic_jk_kernel<float><<<grid, 32 * warps, bytes * warps, s>>>(pv, cl);
+        eri_generic_jk_kernel<float, false><<<grid, 32 * warps, bytes * warps, s>>>(pv, cl, nullptr);
     else
-        eri_generic_jk_kernel<double><<<grid, 32 * warps, bytes * warps, s>>>(pv, cl);
+        eri_generic_jk_kernel<double, false><<<grid, 32 * warps, bytes * warps, s>>>(pv, cl, nullptr);
     TLNO_CUDA(cudaGetLastError());
 }
 

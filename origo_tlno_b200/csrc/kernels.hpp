@@ -21,6 +21,11 @@ void ensure_device_tables();
 
 // Shared-memory bytes per warp of the generic kernel for a class.
 int generic_warp_bytes(int la, int lb, int lc, int ld);
+// Shared memory a block of the warp-per-quartet kernels can take, and whether
+// one warp's region of a class is larger (it then lives in global scratch
+// allocated for the launch).
+constexpr int kMaxWarpSmem = 227 * 1024;
+bool generic_needs_scratch(int la, int lb, int lc, int ld);
 // Builds the pair projectors of every pair with an offset >= 0.
 void launch_pair_projectors(const int* pair_A, const int* pair_B, const double* shell_xyz, const int* shell_L,
                             const long long* off, int n_pairs, double* out, cudaStream_t s);

@@ -88,6 +88,10 @@ extern "C" int tlno_gpu_eri_blocks_noalloc(tlno_gpu_context* ctx, int n_quartets
                 pnp.push_back(static_cast<int>(prim.size() - before));
             }
             const int la = b.shells[sh[0]].L, lb = b.shells[sh[1]].L, lc = b.shells[sh[2]].L, ld = b.shells[sh[3]].L;
+            if (generic_needs_scratch(la, lb, lc, ld))
+                throw Error(TLNO_GPU_E_INVALID,
+                            "tlno_gpu_eri_blocks_noalloc: a quartet with this many g and f shells needs more than a "
+                            "block's shared memory; use tlno_gpu_eri_blocks");
             by_class[((la * 5 + lb) * 5 + lc) * 5 + ld].push_back(q);
         }
         std::vector<int> qb, qk, cls_begin, cls_key;
