@@ -146,5 +146,11 @@ def test_threads_build_beside_each_other():
         t.join()
     assert not failed, failed
     assert max(worst) < 1e-12
-    for w in work:
-        w[0].close()
+    # a captured graph outlives the thread, and its streams, that captured it
+    for ctx, D, ref, d, J, K in work:
+        J.zero_(), K.zero_()
+        torch.cuda.synchronize()
+        ctx.graph_launch()
+        ctx.synchronize()
+        assert max(_maxabs(J.cpu().numpy(), ref["J"]), _maxabs(K.cpu().numpy(), ref["K"])) < 1e-12
+        ctx.close()
