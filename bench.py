@@ -640,7 +640,7 @@ def run_native(args):
     dom_tag = f"({cdom['la']}{cdom['lb']}|{cdom['lc']}{cdom['ld']})"
     traffic, traffic_key = _profiled_traffic(args.config, dom_tag)
     # kernels per build: one per class combination and precision pass, the
-    # max|D| reduction (mixed) and the two final symmetrisations
+    # clearing pass, the max|D| reduction (mixed) and the final symmetrisation
     n_cls = sum(1 for cb in combos if cb["n_tiles"] > 0)
     launches = 2 * n_cls + 3
 

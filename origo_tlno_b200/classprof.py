@@ -98,7 +98,7 @@ def main(argv=None) -> int:
     for i, c in enumerate(ctx.combos()):
         if want and tag(c) not in want:
             continue
-        row = {"index": i, "class": tag(c), "kernel": "compile-time" if c["fast"] else "warp-per-quartet",
+        row = {"index": i, "class": tag(c), "kernel": "compile-time" if c["fast"] else "block- or warp-per-quartet",
                "tiles": c["n_tiles"], "quartets": c["quartets"], "prim_quartets": c["prim_quartets"],
                "flops_model": c["flops"]}
         if not a.plan_only:

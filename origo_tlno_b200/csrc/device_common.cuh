@@ -163,7 +163,8 @@ __device__ __forceinline__ void rys_root(int N, R T, int i, R& root, R& weight) 
 // 5 FP64 operations and no special-case branch.  With the asymptotic form built
 // on it (one rsqrt_pos instead of a division and a square root), which most warps
 // run for some lane: six light classes of 91 waters FP64 208 -> 184 ms, FP32
-// 138 -> 118 ms.
+// 138 -> 118 ms.  Relative error up to 1.4e-16 in FP64 (CUDA's rsqrt is specified
+// to 2.2e-16), 1.2e-7 in FP32, the instruction's own.
 __device__ __forceinline__ double rsqrt_pos(double x) {
     double y;
     asm("rsqrt.approx.ftz.f64 %0, %1;" : "=d"(y) : "d"(x));

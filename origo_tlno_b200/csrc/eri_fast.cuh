@@ -28,8 +28,8 @@
 //
 // What bounds it (40 waters, (ps|ss) FP64, ncu): about 130 issued instructions
 // per primitive quartet of a warp, 55 of them FP64, at 16 resident warps; issue
-// 43%, FP64 pipe 36%, the rest waits on FP64 latency (2.7 cycles per issue) and
-// L1/L2 loads (3.8); with digestion the L1 data pipe is at 76% of its wavefront
+// 42%, FP64 pipe 37%, the rest waits on FP64 latency (2.7 cycles per issue) and
+// L1/L2 loads (4.0); with digestion the L1 data pipe is at 76% of its wavefront
 // rate (scattered atomics and density copies).
 //
 // Arithmetic follows the reference's producer: contracted radial

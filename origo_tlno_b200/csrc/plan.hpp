@@ -12,8 +12,8 @@
 namespace tlno_gpu {
 
 // Device memory a plan may spend on pair-projector tables.  A table saves the
-// block-per-quartet kernels the maps of every quartet (f-shell 14 atoms, the 18
-// classes without a compile-time kernel: 12.9 ms with it, 160 ms in the
+// block-per-quartet kernels the maps of every quartet (f-shell 14 atoms, the 19
+// f classes without a compile-time kernel: 12.9 ms with it, 160 ms in the
 // warp-per-quartet kernel, which builds them per quartet), so it may take up to
 // a tenth of the device.
 constexpr long long kMaxProjectorBytes = 16LL << 30;
