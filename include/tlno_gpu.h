@@ -275,7 +275,8 @@ int tlno_gpu_boys(int device, int n, int maxn, const double* x, double* out);
  * kernels: 0 = FP64 tables (the reference's 0.01-grid interpolant),
  * 1 = FP32 tables, 2 = the FP32 interval polynomials of the mixed-precision
  * kernels (nroots <= 3); 3 and 4 = what the compile-time kernels run in FP64 and
- * in their FP32 pass (nroots <= 5; a NaN argument is passed on to them). */
+ * in their FP32 pass (nroots <= 5); 5 and 6 = modes 0 and 1.  Modes 3 to 6 pass
+ * a NaN argument on to the kernels' code. */
 int tlno_gpu_rys(int device, int n, int nroots, const double* T, double* roots, double* weights,
                  int fp32);
 /* 1/sqrt(x) as the ERI kernels evaluate it, at n positive normal arguments

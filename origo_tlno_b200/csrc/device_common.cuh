@@ -138,7 +138,8 @@ template <> struct RysTab<float> {
 
 template <typename R>
 __device__ __forceinline__ void rys_root(int N, R T, int i, R& root, R& weight) {
-    if (T >= R(c_tabs.tmax[N])) {
+    // the table only for T < tmax: a NaN converts to INT_MIN from FP64
+    if (!(T < R(c_tabs.tmax[N]))) {
         const R inv = R(1) / T;
         root = R(c_tabs.h2[N][i]) * inv;
         weight = R(c_tabs.hw[N][i]) * sqrt(inv);

@@ -838,7 +838,7 @@ void launch_rsqrt_test(const double* x, int n, int mode, double* out, cudaStream
 
 void launch_rys_test(const double* t, int n, int nroots, int fp32, double* roots, double* weights,
                      cudaStream_t s) {
-    if (fp32 >= 3) {
+    if (fp32 == 3 || fp32 == 4) {
         const int g = (n + 127) / 128;
         switch (nroots) {
             case 1: rys_fast_test_kernel<1><<<g, 128, 0, s>>>(t, n, fp32, roots, weights); break;
@@ -851,7 +851,7 @@ void launch_rys_test(const double* t, int n, int nroots, int fp32, double* roots
         TLNO_CUDA(cudaGetLastError());
         return;
     }
-    if (fp32 >= 2) {
+    if (fp32 == 2) {
         const int g = (n + 127) / 128;
         switch (nroots) {
             case 1: rys_interval_test_kernel<1><<<g, 128, 0, s>>>(t, n, fp32, roots, weights); break;
@@ -862,7 +862,7 @@ void launch_rys_test(const double* t, int n, int nroots, int fp32, double* roots
         TLNO_CUDA(cudaGetLastError());
         return;
     }
-    if (fp32)
+    if (fp32 == 1 || fp32 == 6)
         rys_test_kernel<float><<<(n + 127) / 128, 128, 0, s>>>(t, n, nroots, roots, weights);
     else
         rys_test_kernel<double><<<(n + 127) / 128, 128, 0, s>>>(t, n, nroots, roots, weights);

@@ -523,7 +523,8 @@ def boys(x, maxn: int, device: int = 0) -> np.ndarray:
     return out
 
 
-RYS_PATHS = {"fp64_table": 0, "fp32_table": 1, "fp32_interval": 2, "fp64_fast": 3, "fp32_fast": 4}
+RYS_PATHS = {"fp64_table": 0, "fp32_table": 1, "fp32_interval": 2, "fp64_fast": 3, "fp32_fast": 4,
+             "fp64_table_any": 5, "fp32_table_any": 6}
 
 
 def rys_roots(T, nroots: int, fp32: bool = False, device: int = 0, path: Optional[str] = None):
